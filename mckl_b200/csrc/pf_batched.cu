@@ -321,14 +321,33 @@ struct __align__(32) ScoreTau {
 struct ScoreArgs {
     uint64_t nmax;
     double *xb;            // nmax per CTA: the cloud at t before its resampling
-    double2 *xw;           // 2 x nmax per CTA: (x_j, lw_j) of the clouds at t - 1 and t, lw_j = log W_j -
-                           // log(rep_j + 1), so that a backward draw reads one 16-byte pair
-    uint32_t *rep, *anc;   // nmax per CTA: copies of each particle at t - 1, parent of each slot
+    double2 *xw;           // nmax per CTA (in shared memory where it fits): (x_j, lw_j) of the cloud at t - 1,
+                           // lw_j = log W_j - log(rep_j + 1), so that a backward draw reads one 16-byte pair
+    uint32_t *anc;         // nmax per CTA (in shared memory where it fits): parent of each slot at t - 1
     ScoreTau *tau;         // 2 x nmax per CTA
     double *score;         // 3 per filter
 };
 
-template <int THREADS>
+// log(u) < lr for u = (w + 1/2) 2^-32, as the double logarithm decides it.
+// The single-precision logarithm of u is within 1e-5 of log u (rounding u:
+// 2^-23 relative; __logf: 2^-21.4 absolute for u in [0.5, 1], 3 ulps of at most
+// 23 below), so it decides whenever lr is further away than that (rounding lr
+// to float is below 2e-6 for |lr| <= 32); a NaN goes to the double comparison.
+__device__ __forceinline__ bool log_less(uint32_t w, double lr)
+{
+    const float u = __fmul_rn(__fadd_rn(__uint2float_rn(w), 0.5f), 0x1p-32f);
+    const float d = __fsub_rn(__double2float_rn(lr), __logf(u));
+    if (fabsf(d) > 1e-4f) return d > 0.0f;
+    return log((static_cast<double>(w) + 0.5) * 0x1p-32) < lr;
+}
+
+// What bounds it: the latency of the backward draws' random reads.  The
+// proposals of a particle's eight moves do not depend on the chain's state, so
+// all of their reads are in flight together; where the cloud (16 bytes a
+// particle) and the slots' parents fit in shared memory they are read from
+// there.  The acceptance tests take a double logarithm only where a
+// single-precision one cannot decide.
+template <int THREADS, bool SMEM>
 __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *filt, const int *order, int nf,
     const double *y, int T, double threshold, double *xa, double *xb, double *lw, uint32_t *scanS, uint32_t *epos,
     double *loglik, uint32_t *nresampled, int *queue, ScoreArgs A)
@@ -339,8 +358,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *fi
     __shared__ int sh_f;
     const uint64_t slot = blockIdx.x, nm = A.nmax;
     double *xnow = A.xb + slot * nm;
-    double2 *xwb[2] = {A.xw + slot * 2 * nm, A.xw + slot * 2 * nm + nm};
-    uint32_t *rep = A.rep + slot * nm, *anc = A.anc + slot * nm;
+    extern __shared__ __align__(16) unsigned char score_dyn[];
+    // the cloud at t - 1 that the backward draws read at random: one buffer,
+    // rewritten behind a barrier once every draw of the step is done
+    double2 *xw = SMEM ? reinterpret_cast<double2 *>(score_dyn) : A.xw + slot * nm;
+    uint32_t *anc = SMEM ? reinterpret_cast<uint32_t *>(score_dyn + nm * sizeof(double2)) : A.anc + slot * nm;
     ScoreTau *taub[2] = {A.tau + slot * 2 * nm, A.tau + slot * 2 * nm + nm};
     while (true) {
         if (threadIdx.x == 0) {
@@ -366,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *fi
         for (uint64_t p = threadIdx.x; p < N; p += THREADS) {
             const double x0 = run.xc[p];
             const double v = x0 * x0 * isd02 - 1.0;
-            xwb[0][p] = make_double2(x0, 0.0);
+            xw[p] = make_double2(x0, 0.0);
             taub[0][p] = ScoreTau{v * phi / q0, v / sx, 0.0, 0.0};
         }
         __syncthreads();
@@ -375,8 +397,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *fi
         // their own parents (anc = identity, rep = 1) and the arrays are not read
         bool resampled = false;
         for (int t = 1; t <= T; ++t) {
-            const double2 *xwp = xwb[(t - 1) & 1];
-            double2 *xwn = xwb[t & 1];
             run.rec_x = xnow;  // the step records its cloud before resampling
             const bool res = run.step(t, yf[t], shd, shd, shu, shj);
             run.rec_x = nullptr;
@@ -387,35 +407,43 @@ __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *fi
             for (uint64_t i = threadIdx.x; i < N; i += THREADS) {
                 const double xi = xnow[i];
                 uint32_t J = resampled ? anc[i] : static_cast<uint32_t>(i);
-                const double2 pJ = xwp[J];
-                double xJ = pJ.x;
-                double dJ = xi - phi * xJ;
-                double lJ = pJ.y;
-                double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-#pragma unroll 1
+                // The eight proposals depend only on the counters, so all of
+                // their reads are issued before the first acceptance test.
+                // k in [0, 2N): the ancestor of slot k, or particle k - N
+                uint32_t jp[8], wu[8];
+#pragma unroll
                 for (int b = 0; b < 4; ++b) {
                     uint32_t wd[4];
                     gb.block(Ctr{{i, static_cast<uint64_t>(t) | (static_cast<uint64_t>(b) << 32), 0, 0}}, wd);
 #pragma unroll
                     for (int m = 0; m < 2; ++m) {
-                        // k in [0, 2N): the ancestor of slot k, or particle k - N
                         const uint32_t k =
                             static_cast<uint32_t>((static_cast<uint64_t>(wd[2 * m]) * (2ull * N32)) >> 32);
-                        const uint32_t jp = k < N32 ? (resampled ? anc[k] : k) : k - N32;
-                        const double2 pp = xwp[jp];
-                        const double dp = xi - phi * pp.x;
-                        const double lp = pp.y;
-                        // log of the acceptance ratio
-                        const double lr = (dJ * dJ - dp * dp) * hsx2 + lp - lJ;
-                        const double u = (static_cast<double>(wd[2 * m + 1]) + 0.5) * 0x1p-32;
-                        if (log(u) < lr) {
-                            J = jp;
-                            xJ = pp.x;
-                            dJ = dp;
-                            lJ = lp;
-                        }
+                        wu[2 * b + m] = wd[2 * m + 1];
+                        jp[2 * b + m] = k < N32 ? (resampled ? anc[k] : k) : k - N32;
                     }
-                    if (b == 1 || b == 3) {  // the states after moves 4 and 8
+                }
+                const double2 pJ = xw[J];
+                double2 pp[8];
+#pragma unroll
+                for (int m = 0; m < 8; ++m) pp[m] = xw[jp[m]];
+                double xJ = pJ.x;
+                double dJ = xi - phi * xJ;
+                double lJ = pJ.y;
+                double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const double dp = xi - phi * pp[m].x;
+                    const double lp = pp[m].y;
+                    // log of the acceptance ratio
+                    const double lr = (dJ * dJ - dp * dp) * hsx2 + lp - lJ;
+                    if (log_less(wu[m], lr)) {
+                        J = jp[m];
+                        xJ = pp[m].x;
+                        dJ = dp;
+                        lJ = lp;
+                    }
+                    if (m == 3 || m == 7) {  // the states after moves 4 and 8
                         const ScoreTau tJ = tp[J];
                         a0 += tJ.a0 + dJ * xJ * isx2;
                         a1 += tJ.a1 + (dJ * dJ * isx2 - 1.0) / sx;
@@ -449,11 +477,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *fi
                 for (uint64_t p = threadIdx.x; p < N; p += THREADS) {
                     const uint32_t b = run.sS[p], e = p + 1 < N ? run.sS[p + 1] : ne;
                     const uint32_t c = (anc[p] == p ? 1u : 0u) + (e - b);
-                    rep[p] = c;
-                    xwn[p] = make_double2(xnow[p], run.st.l[p] - log(static_cast<double>(c) + 1.0));
+                    xw[p] = make_double2(xnow[p], run.st.l[p] - log(static_cast<double>(c) + 1.0));
                 }
             } else {
-                for (uint64_t p = threadIdx.x; p < N; p += THREADS) xwn[p] = make_double2(xnow[p], run.st.l[p]);
+                for (uint64_t p = threadIdx.x; p < N; p += THREADS) xw[p] = make_double2(xnow[p], run.st.l[p]);
             }
             __syncthreads();
         }
@@ -580,27 +607,44 @@ int pf_adjoint_launch(const BatchedArgs &a, const int *order, int nf, int thread
     }
 }
 
-template <int THREADS>
+// The score's block shape is its own: 512 threads (128 registers: the eight
+// proposals of a particle are in flight at once), one CTA per SM.  256 filters
+// x 8192 particles x 100 steps (one B200): 57.7 ms with the dependent reads and
+// 256-thread CTAs; with the independent reads 36.7 / 28.1 / 37.0 ms at 256
+// threads x 1 / 2 / 4 CTAs per SM, 25.2 / 26.8 at 512 x 1 / 2, 26.5 at 1024 x 1;
+// 21.9 ms at 512 x 1 with the cloud in shared memory.
+constexpr int kScoreThreads = 512;
+// shared memory left for the cloud beside the step's own
+constexpr size_t kScoreDyn = 227 * 1024 - 4 * shj_words<kScoreThreads>() - 1024;
+constexpr size_t kScoreCloudBytes = sizeof(double2) + sizeof(uint32_t);
+
+// Whether a cloud of n particles is kept in shared memory (up to about 10 400).
+bool score_in_smem(uint64_t n)
+{
+    return n * kScoreCloudBytes <= kScoreDyn;
+}
+
+template <bool SMEM>
 int score_one(const BatchedArgs &a, const int *order, int nf, int *queue, const ScoreArgs &A, int ctas,
     cudaStream_t s)
 {
-    k_pf_score<THREADS><<<ctas, THREADS, 0, s>>>(a.filt, order, nf, a.y, a.T, a.threshold,
+    const int dyn = SMEM ? static_cast<int>(A.nmax * kScoreCloudBytes) : 0;
+    if (dyn)
+        MB_CUDA(cudaFuncSetAttribute(k_pf_score<kScoreThreads, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            static_cast<int>(kScoreDyn)));
+    k_pf_score<kScoreThreads, SMEM><<<ctas, kScoreThreads, dyn, s>>>(a.filt, order, nf, a.y, a.T, a.threshold,
         static_cast<double *>(a.xa), static_cast<double *>(a.xb), static_cast<double *>(a.lw), a.scanS, a.epos,
         a.loglik, a.nresampled, queue, A);
     MB_LAUNCH_CHECK();
     return MCKL_B200_OK;
 }
 
-int pf_score_launch(const BatchedArgs &a, const int *order, int nf, int threads, int *queue, const ScoreArgs &A,
-    int ctas, cudaStream_t s)
+int pf_score_launch(const BatchedArgs &a, const int *order, int nf, int *queue, const ScoreArgs &A, int ctas,
+    cudaStream_t s)
 {
     MB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
-    switch (threads) {
-        case 128: return score_one<128>(a, order, nf, queue, A, ctas, s);
-        case 256: return score_one<256>(a, order, nf, queue, A, ctas, s);
-        case 512: return score_one<512>(a, order, nf, queue, A, ctas, s);
-        default: return score_one<1024>(a, order, nf, queue, A, ctas, s);
-    }
+    return score_in_smem(A.nmax) ? score_one<true>(a, order, nf, queue, A, ctas, s)
+                                 : score_one<false>(a, order, nf, queue, A, ctas, s);
 }
 
 int pf_batched_launch(const BatchedArgs &a, const int *order, int nf, int threads, int ctas_per_sm, int *queue,
@@ -1038,9 +1082,9 @@ int mckl_b200_batched_score(mckl_b200_batched_t *b, double *loglik, double *scor
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int ctas = std::max(1, std::min(b->F, sms));
-    const uint64_t nm = b->nmax;
-    const size_t need = align256(ctas * nm * 8) + align256(ctas * 2 * nm * sizeof(double2)) +
-                        2 * align256(ctas * nm * 4) + align256(ctas * 2 * nm * sizeof(ScoreTau)) +
+    const uint64_t nm = b->nmax, ng = score_in_smem(nm) ? 0 : nm;  // ng: particles of the cloud in global memory
+    const size_t need = align256(ctas * nm * 8) + align256(ctas * ng * sizeof(double2)) +
+                        align256(ctas * ng * 4) + align256(ctas * 2 * nm * sizeof(ScoreTau)) +
                         align256(static_cast<size_t>(b->F) * 24);
     if (b->score_bytes < need) {
         if (b->score_mem) cudaFree(b->score_mem);
@@ -1061,12 +1105,11 @@ int mckl_b200_batched_score(mckl_b200_batched_t *b, double *loglik, double *scor
     ScoreArgs A{};
     A.nmax = nm;
     A.xb = reinterpret_cast<double *>(take(ctas * nm * 8));
-    A.xw = reinterpret_cast<double2 *>(take(ctas * 2 * nm * sizeof(double2)));
-    A.rep = reinterpret_cast<uint32_t *>(take(ctas * nm * 4));
-    A.anc = reinterpret_cast<uint32_t *>(take(ctas * nm * 4));
+    A.xw = reinterpret_cast<double2 *>(take(ctas * ng * sizeof(double2)));
+    A.anc = reinterpret_cast<uint32_t *>(take(ctas * ng * 4));
     A.tau = reinterpret_cast<ScoreTau *>(take(ctas * 2 * nm * sizeof(ScoreTau)));
     A.score = reinterpret_cast<double *>(take(static_cast<size_t>(b->F) * 24));
-    int rc = pf_score_launch(b->a, b->order, b->F, b->threads, b->queue, A, ctas, s);
+    int rc = pf_score_launch(b->a, b->order, b->F, b->queue, A, ctas, s);
     if (rc != MCKL_B200_OK) return rc;
     if (loglik) MB_CUDA(cudaMemcpyAsync(loglik, b->a.loglik, b->F * 8, cudaMemcpyDeviceToHost, s));
     MB_CUDA(cudaMemcpyAsync(score, A.score, static_cast<size_t>(b->F) * 24, cudaMemcpyDeviceToHost, s));
