@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "resample.cuh"
+#include "smc_coop_host.cuh"
 #include "weight.cuh"
 
 namespace mckl_b200 {
@@ -184,6 +185,16 @@ extern "C" int mckl_b200_pf_ar1_plain_f64(size_t N, size_t T, const double *y, d
     MB_CHECK_ARG(scheme >= 0 && scheme <= 5, "scheme must be 0..5");
     MB_CHECK_ARG(sy > 0 && sd0 > 0, "sy and sd0 must be positive");
     cudaStream_t s = as_stream(stream);
+    {
+        // a cloud that fits the chip at once: every step in one kernel
+        const CoopFilter f{N, T, y, phi, sx, sd0, -std::log(sy) - 0.5 * std::log(2 * 3.14159265358979323846),
+            0.5 / (sy * sy), 1.0 / static_cast<double>(N), static_cast<double>(N) * threshold, {mkey[0], mkey[1]},
+            {rkey[0], rkey[1]}, scheme, x_dev, W_dev, anc_dev};
+        uint64_t nt = 0;
+        const int cc = coop_filter(f, loglik, ess_hist, resampled, &nt, s);
+        if (cc == MCKL_B200_OK) g_last_ties = nt;
+        if (cc != kCoopNo) return cc;
+    }
     // work buffers: eps, ll, rep, idx, result words
     const size_t wsz = weight_scratch_bytes(N), rsz = resample_scratch_bytes(N, N), isz = rep_index_scratch_bytes(N, N);
     const size_t buf = 5 * align256(N * sizeof(double)) + 512 + align256((T + 1) * sizeof(double));

@@ -24,6 +24,7 @@
 #include "crmath.cuh"
 #include "fold.cuh"
 #include "resample.cuh"
+#include "smc_coop_host.cuh"
 #include "transforms.cuh"
 
 namespace mckl_b200 {
@@ -702,6 +703,53 @@ template int select_dev<double>(uint64_t, uint64_t, uint64_t, const uint64_t *, 
 template int select_dev<float>(uint64_t, uint64_t, uint64_t, const uint64_t *, const float *, float *,
     cudaStream_t);
 
+// The cooperative path (smc_coop.cuh): the engine's canonical uniforms, then
+// one kernel.  The stratified and sorted sequences of the residual schemes use
+// as many uniforms as the weights leave, so up to M are drawn and the engine
+// moves by the number used.
+static int resample_coop(int scheme, uint64_t N, uint64_t M, mckl_b200_engine_t &e, const double *W, uint64_t *rep,
+    cudaStream_t s)
+{
+    if (!coop_fits(std::max(N, M))) return kCoopNo;
+    const bool one = scheme % 3 == 2;
+    double *canon = static_cast<double *>(scratch(10, std::max<uint64_t>(one ? 1 : M, 1) * sizeof(double), s));
+    if (!canon) {
+        set_error("scratch allocation failed");
+        return MCKL_B200_ERR_NOMEM;
+    }
+    Ctr B;
+    uint32_t off;
+    next_position(e, B, off);
+    const uint64_t n = one ? 1 : M;
+    int rc = with_gen(e, [&](auto g) {
+        using G = decltype(g);
+        if (n == 0) return static_cast<int>(MCKL_B200_OK);
+        k_canonical<G><<<cap_grid(n, 256), 256, G::kDynSmem, s>>>(g, B, off, n, canon);
+        MB_LAUNCH_CHECK();
+        return static_cast<int>(MCKL_B200_OK);
+    });
+    if (rc != MCKL_B200_OK) return rc;
+    CoopResult *res = nullptr;
+    rc = coop_resample(scheme, N, M, W, canon, rep, &res, s);
+    if (rc != MCKL_B200_OK) return rc;
+    uint64_t used = M;
+    if (scheme >= 3) {
+        CoopResult h;
+        rc = coop_read(res, &h, s);  // the count of uniforms decides the engine's consumption
+        if (rc != MCKL_B200_OK) return rc;
+        used = h.used;
+    }
+    if (one) {
+        advance_call(e, 1);  // U01Distribution<double>{}(rng): two single-word draws
+        advance_call(e, 1);
+    } else if (used > 0) {
+        // per 1024-chunk: u01_canonical_distribution -> one call of 2 words per value
+        advance_calls(e, used / 1024, 2048);
+        advance_call(e, 2 * (used % 1024));
+    }
+    return MCKL_B200_OK;
+}
+
 }  // namespace mckl_b200
 
 using namespace mckl_b200;
@@ -735,6 +783,8 @@ int mckl_b200_resample(int scheme, size_t N, size_t M, mckl_b200_engine_t *rng, 
     MB_CHECK_ARG(N < (1ull << 31) && M < (1ull << 31), "N and M must be below 2^31");
     if (N == 0) return MCKL_B200_OK;
     cudaStream_t s = as_stream(stream);
+    const int cc = resample_coop(scheme, N, M, *rng, W, rep, s);
+    if (cc != kCoopNo) return cc;
     void *base = scratch(3, resample_scratch_bytes(N, M), s);
     if (!base) {
         set_error("scratch allocation failed");
@@ -748,6 +798,14 @@ int mckl_b200_rep_to_index(size_t N, size_t M, const uint64_t *rep, uint64_t *id
     MB_CHECK_ARG(N == 0 || M == 0 || (rep != nullptr && idx != nullptr), "null pointer");
     MB_CHECK_ARG(N < (1ull << 31) && M < (1ull << 31), "N and M must be below 2^31");
     cudaStream_t s = as_stream(stream);
+    if (N > 0 && M > 0) {
+        CoopResult *res = nullptr;
+        const int cc = coop_rep_to_index(N, M, rep, idx, &res, s);
+        if (cc != kCoopNo) {
+            CoopResult h;
+            return cc == MCKL_B200_OK && res ? coop_read(res, &h, s) : cc;
+        }
+    }
     void *base = scratch(4, rep_index_scratch_bytes(N, M) + 64, s);
     if (!base) {
         set_error("scratch allocation failed");

@@ -91,6 +91,12 @@ void *scratch(int slot, size_t bytes, cudaStream_t stream)
             b.ptr = nullptr;
             return nullptr;
         }
+        // a new buffer's header is zero (the cooperative kernels keep an error word there)
+        if (cudaMemsetAsync(b.ptr, 0, 256, stream) != cudaSuccess) {
+            cudaFreeAsync(b.ptr, stream);
+            b.ptr = nullptr;
+            return nullptr;
+        }
         b.bytes = want;
     }
     return b.ptr;

@@ -17,6 +17,7 @@
 #include "common.cuh"
 #include "crmath.cuh"
 #include "fold.cuh"
+#include "smc_coop_host.cuh"
 #include "weight.cuh"
 
 namespace mckl_b200 {
@@ -203,6 +204,19 @@ static int weight_call(size_t N, double *W, const double *v, int add_log, double
     MB_CHECK_ARG(N > 0, "N must be positive");
     MB_CHECK_ARG(W != nullptr && v != nullptr, "null pointer");
     cudaStream_t s = as_stream(stream);
+    CoopResult *cr = nullptr;
+    const int cc = coop_weight(N, W, v, add_log, &cr, s);
+    if (cc != kCoopNo) {
+        if (cc != MCKL_B200_OK) return cc;
+        if (ess || log_nc) {
+            CoopResult h;
+            const int rc = coop_read(cr, &h, s);
+            if (rc != MCKL_B200_OK) return rc;
+            if (ess) *ess = h.ess;
+            if (log_nc) *log_nc = h.log_nc;
+        }
+        return MCKL_B200_OK;
+    }
     void *base = scratch(2, weight_scratch_bytes(N) + 64, s);
     if (!base) {
         set_error("weight scratch allocation failed");
