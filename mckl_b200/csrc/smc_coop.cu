@@ -51,7 +51,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_weight(Global g, unsign
         }
     }
     WeightOut r;
-    if (!weight_phase<PER>(c, tm.v, tm.q, N, m, r)) return;
+    Approx ap;
+    if (!weight_phase<PER>(c, tm.v, tm.q, N, m, r, ap)) return;
     const double inv = __ddiv_rn(1.0, r.accw);
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_resample(Global g, unsi
     __syncthreads();
     uint64_t R;
     if (!resample_phase<PER>(c, tm.v, tm.q, N, M, scheme, [canon](uint64_t j) { return __ldg(canon + j); },
-            [W](uint64_t i) { return W[i]; }, ubuf, &R, nullptr))
+            [W](uint64_t i) { return W[i]; }, ubuf, nullptr, &R, nullptr))
         return;
     __syncthreads();
 #pragma unroll 2
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
     bool flat = true;    // the weights are all equal
     int cur = 0;
     double *x = a.xb[0];
+    Approx ap;           // of the step's terms
     tile_normals<PER>(c, gm, N, 0, a.sd0, [&](uint32_t o, double e) { x[base + o] = e; });
     __syncthreads();
     for (uint64_t t = 0; t <= a.T; ++t) {
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
             cur ^= 1;
             x = xn;
             WeightOut r;
-            if (!weight_phase<PER>(c, tm.v, tm.q, N, m, r)) return;
+            if (!weight_phase<PER>(c, tm.v, tm.q, N, m, r, ap)) return;
             accw = r.accw;
             ess = r.ess;
             flat = false;
@@ -262,6 +264,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
             tm.v[at<PER>(k)] = w;
             if ((a.scheme >= 3 || a.scheme == 0) && i < N) a.W[i] = w;
         }
+        // the weights' approximate sums are the terms' times 1 / accw: a few
+        // roundings more, which the classification's margin holds many times
+        const Approx apw{__dmul_rn(inv, ap.A), __dmul_rn(inv, ap.own), __dmul_rn(inv, ap.M)};
         uint64_t R;
         const uint64_t rp = rpos;
         if (!resample_phase<PER>(c, tm.v, tm.q, N, N, a.scheme,
@@ -271,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
                     gr.block(Ctr{{(w >> 2) + 1, 0, 0, 0}}, blk);
                     return (w & 2) ? u01_canonical2(blk[2], blk[3]) : u01_canonical2(blk[0], blk[1]);
                 },
-                [&a](uint64_t i) { return a.W[i]; }, a.ubuf, &R, &ties))
+                [&a](uint64_t i) { return a.W[i]; }, a.ubuf, flat ? nullptr : &apw, &R, &ties))
             return;
         rpos += a.scheme % 3 == 2 ? 2 : 2 * R;
         __syncthreads();

@@ -248,6 +248,45 @@ __device__ __forceinline__ void scan_sum_max(Ctx &c, double v, double m, double 
     em = warp > 0 ? fmax(bm, pm) : pm;
 }
 
+// Maximum over the warp of nonnegative doubles (their bits order as unsigned
+// integers: the high words first, then the low words among the largest).
+__device__ __forceinline__ double warp_max_nonneg(double v)
+{
+    const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double(static_cast<int>(mh), static_cast<int>(ml));
+}
+
+// Exclusive sums of nonnegative values (formed without a subtraction) and the
+// total; em: the maximum over the warps before this one, tm over all.
+__device__ __forceinline__ void scan_sum(Ctx &c, double v, double m, double &es, double &em, double &ts, double &tm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double is = warp_inclusive_sum(v), wmx = warp_max_nonneg(m);
+    double ps = __shfl_up_sync(0xffffffffu, is, 1);
+    if (lane == 0) ps = 0.0;
+    c.flip ^= 1;
+    unsigned long long(*buf)[kWarps] = c.sh->scr[c.flip];
+    if (lane == 31) {
+        buf[0][warp] = dbits(is);
+        buf[1][warp] = dbits(wmx);
+    }
+    __syncthreads();
+    double ws = lane < kWarps ? bitsd(buf[0][lane]) : 0.0;
+    const double wm = lane < kWarps ? bitsd(buf[1][lane]) : 0.0;
+#pragma unroll
+    for (int o = 1; o < kWarps; o <<= 1) {
+        const double us = __shfl_up_sync(0xffffffffu, ws, o);
+        if (lane >= o) ws += us;
+    }
+    const double bs = __shfl_sync(0xffffffffu, ws, warp > 0 ? warp - 1 : 0);
+    ts = __shfl_sync(0xffffffffu, ws, kWarps - 1);
+    tm = warp_max_nonneg(wm);
+    em = warp_max_nonneg(lane < warp ? wm : 0.0);
+    es = warp > 0 ? bs + ps : ps;
+}
+
 // Exclusive sums of two 64-bit integers, and the totals.
 __device__ __forceinline__ void scan_two(Ctx &c, long long a, long long b, long long &ea, long long &eb,
     long long &ta, long long &tb)
@@ -360,10 +399,28 @@ __device__ __forceinline__ void classify_tile(const Get &get, long long *s_q, ui
     {
         const double Aend = __dadd_rn(Abefore, own);
         const double m = 2.0 * static_cast<double>(i0 + PER) + 2.0 * static_cast<double>(T) + 160.0;
-        const double lo = fmax(__dsub_rn(Abefore, m * ulp_of(Abefore)), Mbefore);
-        const double hi = __dadd_rn(Aend, m * ulp_of(Aend));
-        const int e = biased_exp(lo);
-        if (lo > 0.0 && e != 0x7ff && biased_exp(hi) == e) fast = e;
+        const double low = __dsub_rn(Abefore, m * ulp_of(Abefore)), hi = __dadd_rn(Aend, m * ulp_of(Aend));
+        const auto certain = [hi](double lo) {
+            const int e = biased_exp(lo);
+            return lo > 0.0 && e != 0x7ff && biased_exp(hi) == e ? e : -1;
+        };
+        fast = certain(fmax(low, Mbefore));
+        if (__any_sync(0xffffffffu, fast < 0)) {
+            // the largest term of the warp's threads before this one, too
+            const int lane = threadIdx.x & 31;
+            double mx = 0.0;
+#pragma unroll 1
+            for (int k = 0; k < PER; ++k)
+                if (i0 + k < n) mx = fmax(mx, get(k));
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double u = __shfl_up_sync(0xffffffffu, mx, o);
+                if (lane >= o) mx = fmax(mx, u);
+            }
+            mx = __shfl_up_sync(0xffffffffu, mx, 1);
+            if (lane > 0) Mbefore = fmax(Mbefore, mx);
+            fast = certain(fmax(low, Mbefore));
+        }
     }
     // A warp whose threads are all certain of their binades, away from the end
     // of the array: the increments alone.  An event sends the warp through the
@@ -552,18 +609,17 @@ __device__ __noinline__ bool fold_chain(Ctx &c, double *s_v, long long *s_q, uin
     return true;
 }
 
-// ---- the exact left fold of n values, from 0.  The tile's values are in s_v
-// (0 past n), each written by its own thread.  The last value goes to *total;
-// with PREFIX every partial sum replaces its value in s_v and the one before
-// the thread's first element goes to *before.  What was written to global
-// memory before the call is visible after it (its second exchange carries
-// data).  s_q is overwritten.  False when a wait gave up.
-template <int PER, bool PREFIX>
-__device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint64_t n, double *total,
-    double *before)
+// What the classification needs of a thread: the approximate sum of the
+// elements before its own, its own sum, and a lower bound of the sum before it
+// (the largest term of the warps and tiles before).
+struct Approx {
+    double A, own, M;
+};
+
+// The approximate sums of the values in s_v (0 past n).  False when a wait gave up.
+template <int PER>
+__device__ __forceinline__ bool fold_approx(Ctx &c, const double *s_v, Approx &ap)
 {
-    Shared *sh = c.sh;
-    const uint64_t i0 = (static_cast<uint64_t>(c.tile) * kThreads + threadIdx.x) * PER;
     double own = 0.0, mx = 0.0;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
@@ -571,29 +627,53 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
         own = __dadd_rn(own, x);
         mx = fmax(mx, x);
     }
-    if (threadIdx.x == 0) {
-        sh->elast = -1;
-        sh->elast_all = -1;
-    }
     double ex, em, ts, tm, tpre = 0.0, tpm = 0.0;
-    scan_sum_max(c, own, mx, ex, em, ts, tm);
+    scan_sum(c, own, mx, ex, em, ts, tm);
     if (c.T > 1) {
         unsigned long long x[2] = {dbits(ts), dbits(tm)};
         if (!exchange(c, x, false)) return false;
-        double e2, m2, t0, t1;
-        scan_sum_max(c, bitsd(x[0]), bitsd(x[1]), e2, m2, t0, t1);
-        if (threadIdx.x == c.tile) {
-            sh->tpre = e2;
-            sh->tpmax = m2;
+        if (c.cluster) {
+            const unsigned long long(*xs)[kMaxCluster] = c.sh->xs[c.epoch & 1];
+            for (uint32_t t = 0; t < c.tile; ++t) {
+                tpre += bitsd(xs[0][t]);
+                tpm = fmax(tpm, bitsd(xs[1][t]));
+            }
+        } else {
+            double e2, m2, t0, t1;
+            scan_sum_max(c, bitsd(x[0]), bitsd(x[1]), e2, m2, t0, t1);
+            if (threadIdx.x == c.tile) {
+                c.sh->tpre = e2;
+                c.sh->tpmax = m2;
+            }
+            __syncthreads();
+            tpre = c.sh->tpre;
+            tpm = c.sh->tpmax;
         }
-        __syncthreads();
-        tpre = sh->tpre;
-        tpm = sh->tpmax;
     }
+    ap.A = __dadd_rn(tpre, ex);
+    ap.own = own;
+    ap.M = fmax(tpm, em);
+    return true;
+}
+
+// ---- the exact left fold of n values, from 0.  The tile's values are in s_v
+// (0 past n), each written by its own thread; ap from fold_approx.  The last
+// value goes to *total; with PREFIX every partial sum replaces its value in s_v
+// and the one before the thread's first element goes to *before.  What was
+// written to global memory before the call is visible after it (its exchange
+// carries data).  s_q is overwritten.  False when a wait gave up.
+template <int PER, bool PREFIX>
+__device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint64_t n, const Approx ap,
+    double *total, double *before)
+{
+    Shared *sh = c.sh;
+    const uint64_t i0 = (static_cast<uint64_t>(c.tile) * kThreads + threadIdx.x) * PER;
+    if (threadIdx.x == 0) sh->elast = -1;
+    __syncthreads();
     unsigned win;
     long long qs;
-    classify_tile<PER>([s_v](int k) { return s_v[at<PER>(k)]; }, s_q, i0, n, c.T, __dadd_rn(tpre, ex), own,
-        fmax(tpm, em), &win, &qs, &sh->elast);
+    classify_tile<PER>([s_v](int k) { return s_v[at<PER>(k)]; }, s_q, i0, n, c.T, ap.A, ap.own, ap.M, &win, &qs,
+        &sh->elast);
     long long P, r, qtot, wtot;
     scan_two(c, qs, __popc(win), P, r, qtot, wtot);
     bool over = wtot > static_cast<long long>(c.T == 1 ? kWin : kTileWin);
@@ -635,12 +715,26 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
         if (!exchange(c, x, true)) return false;
         const long long wi = static_cast<long long>(x[1] >> 32);
         const int el = static_cast<int>(static_cast<uint32_t>(x[1])) - 1;
-        long long eq, ew, tq, tw;
-        scan_two(c, static_cast<long long>(x[0]), wi, eq, ew, tq, tw);
+        long long eq = 0, ew = 0, tq = 0, tw = 0;
+        if (c.cluster) {
+            const unsigned long long(*xs)[kMaxCluster] = sh->xs[c.epoch & 1];
+            for (uint32_t t = 0; t < c.T; ++t) {
+                const long long q = static_cast<long long>(xs[0][t]), w = static_cast<long long>(xs[1][t] >> 32);
+                if (t < threadIdx.x) {
+                    eq += q;
+                    ew += w;
+                }
+                tq += q;
+                tw += w;
+            }
+        } else {
+            scan_two(c, static_cast<long long>(x[0]), wi, eq, ew, tq, tw);
+        }
         if (threadIdx.x < c.T) {
             sh->pq[threadIdx.x] = eq;
             sh->pw[threadIdx.x] = static_cast<uint32_t>(ew);
-            if (el >= 0) sh->elast_all = el;
+            // the tile that holds element n - 1 tells its run's binade
+            if (threadIdx.x == (n - 1) / (kThreads * PER)) sh->elast_all = el;
         }
         over = __syncthreads_or(wi > static_cast<long long>(kTileWin)) || tw > static_cast<long long>(kWin);
         W = static_cast<unsigned>(tw);
@@ -710,37 +804,28 @@ __device__ void seg_fold(Ctx &c, long long *s_q, uint32_t len, const Get &get, c
         mx = fmax(mx, x);
     }
     if (i0 == 0) sh->gel[seg] = -1;
-    double is = own, im = mx;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double us = __shfl_up_sync(0xffffffffu, is, o), um = __shfl_up_sync(0xffffffffu, im, o);
-        if (lane >= o) {
-            is += us;
-            im = fmax(im, um);
-        }
-    }
-    double ps = __shfl_up_sync(0xffffffffu, is, 1), pm = __shfl_up_sync(0xffffffffu, im, 1);
-    if (lane == 0) ps = pm = 0.0;
+    const double is = warp_inclusive_sum(own), wmx = warp_max_nonneg(mx);
+    double ps = __shfl_up_sync(0xffffffffu, is, 1);
+    if (lane == 0) ps = 0.0;
     c.flip ^= 1;
     unsigned long long(*buf)[kWarps] = sh->scr[c.flip];
     if (lane == 31) {
         buf[0][warp] = dbits(is);
-        buf[1][warp] = dbits(im);
+        buf[1][warp] = dbits(wmx);
     }
     __syncthreads();
-    double ws = lane < kWarps ? bitsd(buf[0][lane]) : 0.0, wm = lane < kWarps ? bitsd(buf[1][lane]) : 0.0;
+    double ws = lane < kWarps ? bitsd(buf[0][lane]) : 0.0;
+    const double wm = lane < kWarps ? bitsd(buf[1][lane]) : 0.0;
 #pragma unroll
     for (int o = 1; o < SW; o <<= 1) {
-        const double us = __shfl_up_sync(0xffffffffu, ws, o), um = __shfl_up_sync(0xffffffffu, wm, o);
-        if ((lane & (SW - 1)) >= o) {
-            ws += us;
-            wm = fmax(wm, um);
-        }
+        const double us = __shfl_up_sync(0xffffffffu, ws, o);
+        if ((lane & (SW - 1)) >= o) ws += us;
     }
     const bool firstw = (warp & (SW - 1)) == 0;
     const double bs = __shfl_sync(0xffffffffu, ws, firstw ? 0 : warp - 1);
-    const double bm = __shfl_sync(0xffffffffu, wm, firstw ? 0 : warp - 1);
-    const double ex = firstw ? ps : bs + ps, em = firstw ? pm : fmax(bm, pm);
+    // the segment's warps before this one
+    const double em = warp_max_nonneg(lane < warp && lane >= (warp & ~(SW - 1)) ? wm : 0.0);
+    const double ex = firstw ? ps : bs + ps;
     unsigned win;
     long long qs;
     classify_tile<PER>(get, s_q, i0, len, 1, ex, own, em, &win, &qs, &sh->gel[seg]);
@@ -824,7 +909,7 @@ struct WeightOut {
 
 template <int PER>
 __device__ __forceinline__ bool weight_phase(Ctx &c, double *s_w, long long *s_q, uint64_t N, double m,
-    WeightOut &out)
+    WeightOut &out, Approx &ap)
 {
     constexpr uint32_t TILE = kThreads * PER;
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE;
@@ -862,13 +947,13 @@ __device__ __forceinline__ bool weight_phase(Ctx &c, double *s_w, long long *s_q
         if (d < nd) dots[d] = c.sh->gtot[threadIdx.x];
     }
     double accw, before;
-    if (!fold_grid<PER, false>(c, s_w, s_q, N, &accw, &before)) return false;
+    if (!fold_approx<PER>(c, s_w, ap) || !fold_grid<PER, false>(c, s_w, s_q, N, ap, &accw, &before)) return false;
     constexpr int DP = (kMaxTiles * NSEG + kThreads - 1) / kThreads;
     static_assert(DP <= PER, "the dots' increments fit the tile's");
-    if (c.T == 1) {
+    if (c.T <= kMaxCluster) {  // a few
         if (threadIdx.x == 0) {
             double t = 0.0;
-            for (uint32_t j = 0; j < nd; ++j) t = __dadd_rn(t, dots[j]);
+            for (uint32_t j = 0; j < nd; ++j) t = __dadd_rn(t, c.T == 1 ? dots[j] : __ldcg(dots + j));
             c.sh->gtot[0] = t;
         }
         __syncthreads();
@@ -975,16 +1060,18 @@ __device__ __forceinline__ void count_reps(const U &u, uint64_t N, uint32_t R, u
 // ---- ResampleAlgorithm::operator() (resample.cu) from the tile's weights in
 // s_v (0 past N).  canon(j): canonical uniform j of the call's stream; again(i):
 // weight i.  ubuf: global memory for the uniforms of the sorted and stratified
-// sequences.  The counts go to s_q (each in its thread's place), the number of
-// uniforms used to *used.
+// sequences.  known (nullable): fold_approx of the weights.  The counts go to
+// s_q (each in its thread's place), the number of uniforms used to *used.
 template <int PER, class Canon, class Again>
 __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s_q, uint64_t N, uint64_t M,
-    int scheme, const Canon &canon, const Again &again, double *ubuf, uint64_t *used, unsigned long long *ties)
+    int scheme, const Canon &canon, const Again &again, double *ubuf, const Approx *known, uint64_t *used,
+    unsigned long long *ties)
 {
     const uint64_t i0 = (static_cast<uint64_t>(c.tile) * kThreads + threadIdx.x) * PER;
     const int seq = scheme % 3;
     uint64_t R = M;
     double before = 0.0, total, mul = 1.0;
+    Approx ap;
     const double coeff = static_cast<double>(M);
     if (scheme >= 3) {
         long long acc = 0;
@@ -1002,7 +1089,7 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
             scan_two(c, static_cast<long long>(x[0]), 0, e0, e1, t0, t1);
         }
         R = static_cast<uint64_t>(t0) <= M ? M - static_cast<uint64_t>(t0) : 0;
-        if (!fold_grid<PER, false>(c, s_v, s_q, N, &total, &before)) return false;
+        if (!fold_approx<PER>(c, s_v, ap) || !fold_grid<PER, false>(c, s_v, s_q, N, ap, &total, &before)) return false;
         mul = __ddiv_rn(1.0, total);
     }
     *used = R;
@@ -1012,7 +1099,7 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
             const uint64_t j = i0 + k;
             s_v[at<PER>(k)] = j < R ? -__ddiv_rn(dd::log(canon(j)), static_cast<double>(R - j)) : 0.0;
         }
-        if (!fold_grid<PER, true>(c, s_v, s_q, R, &total, &before)) return false;
+        if (!fold_approx<PER>(c, s_v, ap) || !fold_grid<PER, true>(c, s_v, s_q, R, ap, &total, &before)) return false;
 #pragma unroll 1
         for (int k = 0; k < PER; ++k)
             if (i0 + k < R) ubuf[i0 + k] = __dsub_rn(1.0, exp_rn(-s_v[at<PER>(k)]));
@@ -1040,7 +1127,12 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
             }
             s_v[at<PER>(k)] = w;
         }
-        if (!fold_grid<PER, true>(c, s_v, s_q, N - 1, &total, &before)) return false;
+        if (known && scheme < 3) {
+            ap = *known;
+        } else if (!fold_approx<PER>(c, s_v, ap)) {
+            return false;
+        }
+        if (!fold_grid<PER, true>(c, s_v, s_q, N - 1, ap, &total, &before)) return false;
         if (seq == 2) {
             const double delta = __ddiv_rn(1.0, static_cast<double>(R));
             const double ud = __dmul_rn(canon(0), delta);
@@ -1110,8 +1202,16 @@ __device__ __forceinline__ bool index_phase(Ctx &c, double *s_v, long long *s_q,
     }
     unsigned long long x[2] = {static_cast<unsigned long long>(te), static_cast<unsigned long long>(ts)};
     if (!exchange(c, x, true)) return false;
-    long long pe, ps, t0, t1;
-    scan_two(c, static_cast<long long>(x[0]), static_cast<long long>(x[1]), pe, ps, t0, t1);
+    long long pe = 0, ps = 0, t0, t1;
+    if (c.cluster) {
+        const unsigned long long(*xs)[kMaxCluster] = sh->xs[c.epoch & 1];
+        for (uint32_t t = 0; t < c.T && t < threadIdx.x; ++t) {
+            pe += static_cast<long long>(xs[0][t]);
+            ps += static_cast<long long>(xs[1][t]);
+        }
+    } else if (c.T > 1) {
+        scan_two(c, static_cast<long long>(x[0]), static_cast<long long>(x[1]), pe, ps, t0, t1);
+    }
     if (threadIdx.x < c.T) {
         sh->pw[threadIdx.x] = static_cast<uint32_t>(pe);
         sh->pq[threadIdx.x] = ps;
