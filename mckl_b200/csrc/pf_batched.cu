@@ -647,12 +647,41 @@ int pf_score_launch(const BatchedArgs &a, const int *order, int nf, int *queue, 
                                  : score_one<false>(a, order, nf, queue, A, ctas, s);
 }
 
-int pf_batched_launch(const BatchedArgs &a, const int *order, int nf, int threads, int ctas_per_sm, int *queue,
-    cudaStream_t s)
+// The filters that a cluster runs (the first of the sorted ones) and their share
+// of the work: those with more particles than a CTA's even share of all of them
+// (on a CTA alone they would be the tail of the batch), and more than 4096
+// (a step of 4096 takes as long either way).  A cluster's four CTAs get 1 / 1.4 of
+// four CTAs' rate out of a filter: the terms are written and read once more, the
+// totals of the resampling are formed twice, and five cluster barriers wait.
+// One B200, 256 threads x 4 CTAs per SM: 1024 filters, log-uniform in
+// [256, 65536], T = 100: 42.6 ms without, 21.9 / 21.3 / 20.9 / 21.3 / 22.9 with
+// those above 0.5 / 0.75 / 1 / 1.25 / 1.5 shares (clusters of 2 and of 8: 25.4 and
+// 24.8 at one share); 300 filters up to 20000, T = 60: 5.5 -> 3.7; 24 filters up to
+// 8375, T = 58: 1.85 -> 1.26.  4096 filters fill the chip by themselves: 32.6 ms
+// (T = 60) either way, 46 with those above half a share by clusters.
+int joint_filters(const uint64_t *sorted, int nf, int slots, double *share)
+{
+    constexpr double kCost = 1.4;
+    double total = 0.0, joint = 0.0;
+    for (int f = 0; f < nf; ++f) total += static_cast<double>(sorted[f]);
+    const double limit = std::max(static_cast<double>(kJointMin), total / slots);
+    int nj = 0;
+    while (nj < nf && static_cast<double>(sorted[nj]) > limit) joint += static_cast<double>(sorted[nj++]);
+    *share = kCost * joint / (kCost * joint + total - joint);
+    return nj;
+}
+
+int pf_batched_launch(const BatchedArgs &a, const int *order, const uint64_t *sorted, int nf, int threads,
+    int ctas_per_sm, int *queue, cudaStream_t s)
 {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (a.terms) {
+        double share = 0.0;
+        const int nj = joint_filters(sorted, nf, sms * ctas_per_sm, &share);
+        if (nj > 0) return pf_batched_joint_launch(a, order, nj, nf, share, threads, sms * ctas_per_sm, queue, s);
+    }
     bool capped = false;
     int fit = 0;
     int rc = pf_batched_fit(a, threads, ctas_per_sm, &capped, &fit);
@@ -680,6 +709,7 @@ struct mckl_b200_batched {
     cudaGraphExec_t exec = nullptr;
     cudaStream_t graph_stream = nullptr;
     std::vector<mckl_b200::BatchedFilter> hf;  // host copy of the filter table
+    std::vector<uint64_t> sorted;              // particle counts, largest first
     uint64_t nmax = 0;                         // largest particle count
     void *adj_mem = nullptr;                   // adjoint checkpoints and work areas
     size_t adj_bytes = 0;
@@ -780,7 +810,24 @@ int mckl_b200_batched_create(mckl_b200_batched_t **out, size_t F, const size_t *
     const size_t bytes = align256(F * sizeof(BatchedFilter)) + align256(F * (T + 1) * 8) + 2 * align256(total * rs) +
                          2 * align256(total * 4) + align256(F * 8) + align256(F * 4) + align256(F * 4) + 256 +
                          (shadow ? 2 * align256(total * 8) + align256(F * 8) : 0);
-    if (cudaMalloc(&b->mem, bytes) != cudaSuccess) {
+    // working memory of the filters that clusters run, for as many clusters as
+    // the device holds (two per SM at the smallest shape), there are such filters
+    // and 48 MiB allow (all of them up to 65536 particles at the default shape);
+    // without room for it none are
+    uint64_t tunits = 0;  // not monotone in the particles: the pairs of a partial chunk are a unit each
+    size_t large = 0;
+    for (size_t f = 0; f < F; ++f) {
+        tunits = std::max(tunits, joint_units(N[f]));
+        large += N[f] > kJointMin ? 1 : 0;
+    }
+    const int tclusters = b->fp64 || shadow
+        ? 0 : static_cast<int>(std::min<size_t>({large, 2 * 148, (48u << 20) / joint_bytes(tunits)}));
+    const size_t tbytes = tclusters * joint_bytes(tunits);
+    if (tbytes && cudaMalloc(&b->mem, bytes + tbytes) == cudaSuccess) {
+        b->a.terms = static_cast<char *>(b->mem) + bytes;
+        b->a.terms_units = tunits;
+        b->a.terms_clusters = tclusters;
+    } else if (cudaGetLastError(), cudaMalloc(&b->mem, bytes) != cudaSuccess) {
         delete b;
         set_error("batched filter allocation failed");
         return MCKL_B200_ERR_NOMEM;
@@ -815,6 +862,7 @@ int mckl_b200_batched_create(mckl_b200_batched_t **out, size_t F, const size_t *
     MB_CUDA(cudaMemcpy(b->a.y, y, F * (T + 1) * 8, cudaMemcpyHostToDevice));
     MB_CUDA(cudaMemcpy(b->order, order.data(), F * 4, cudaMemcpyHostToDevice));
     b->hf = h;
+    for (int f : order) b->sorted.push_back(N[f]);
     for (size_t f = 0; f < F; ++f) b->nmax = std::max<uint64_t>(b->nmax, N[f]);
     *out = b;
     return MCKL_B200_OK;
@@ -849,7 +897,7 @@ int mckl_b200_batched_get_config(const mckl_b200_batched_t *b, int *threads, int
 int mckl_b200_batched_run(mckl_b200_batched_t *b, void *stream)
 {
     MB_CHECK_ARG(b != nullptr, "null handle");
-    return pf_batched_launch(b->a, b->order, b->F, b->threads, b->ctas_per_sm, b->queue, as_stream(stream));
+    return pf_batched_launch(b->a, b->order, b->sorted.data(), b->F, b->threads, b->ctas_per_sm, b->queue, as_stream(stream));
 }
 
 int mckl_b200_batched_run_graph(mckl_b200_batched_t *b, void *stream)
@@ -860,7 +908,7 @@ int mckl_b200_batched_run_graph(mckl_b200_batched_t *b, void *stream)
         cudaStream_t cap;
         MB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         MB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        const int rc = pf_batched_launch(b->a, b->order, b->F, b->threads, b->ctas_per_sm, b->queue, cap);
+        const int rc = pf_batched_launch(b->a, b->order, b->sorted.data(), b->F, b->threads, b->ctas_per_sm, b->queue, cap);
         cudaGraph_t g = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(cap, &g);
         cudaStreamDestroy(cap);
@@ -900,7 +948,7 @@ int mckl_b200_batched_autotune(mckl_b200_batched_t *b, int max_trials, int *thre
     MB_CUDA(cudaEventCreate(&e0));
     MB_CUDA(cudaEventCreate(&e1));
     // one untimed run first (module load, caches)
-    int rc = pf_batched_launch(b->a, b->order, b->F, 256, 4, b->queue, s);
+    int rc = pf_batched_launch(b->a, b->order, b->sorted.data(), b->F, 256, 4, b->queue, s);
     for (int k = 0; rc == MCKL_B200_OK && k < static_cast<int>(sizeof(cand) / sizeof(cand[0])); ++k) {
         int fit = 0;
         bool capped = false;
@@ -908,7 +956,7 @@ int mckl_b200_batched_autotune(mckl_b200_batched_t *b, int max_trials, int *thre
         if (rc != MCKL_B200_OK) break;
         if (fit < cand[k][1]) continue;  // would not be resident at once
         cudaEventRecord(e0, s);
-        rc = pf_batched_launch(b->a, b->order, b->F, cand[k][0], cand[k][1], b->queue, s);
+        rc = pf_batched_launch(b->a, b->order, b->sorted.data(), b->F, cand[k][0], cand[k][1], b->queue, s);
         cudaEventRecord(e1, s);
         if (rc != MCKL_B200_OK) break;
         if (cudaEventSynchronize(e1) != cudaSuccess) {

@@ -29,9 +29,32 @@ struct BatchedArgs {
     uint32_t *nresampled;
     double *xsa = nullptr, *xsb = nullptr, *lws = nullptr;  // FP64 shadow (FP32 run only)
     double *loglik_shadow = nullptr;
+    char *terms = nullptr;  // working memory of the filters run by clusters (null: none are):
+                            // terms_clusters x joint_bytes(terms_units)
+    uint64_t terms_units = 0;
+    int terms_clusters = 0;
 };
 
-int pf_batched_launch(const BatchedArgs &a, const int *order, int nf, int threads, int ctas_per_sm, int *queue,
-    cudaStream_t s);
+// Units of a filter of n particles with the entry of an odd last one, even.
+inline uint64_t joint_units(uint64_t n)
+{
+    return (n / 1024 * 129 + n % 1024 / 2 + 2) / 2 * 2;
+}
+
+inline size_t joint_bytes(uint64_t units)
+{
+    return units * 40;  // two float4 and a double per unit
+}
+
+// sorted: the filters' particle counts, largest first (host).
+int pf_batched_launch(const BatchedArgs &a, const int *order, const uint64_t *sorted, int nf, int threads,
+    int ctas_per_sm, int *queue, cudaStream_t s);
+// The first nj filters of the order by a cluster of kJointCtas CTAs each, the
+// others by a CTA each (FP32, no shadow); share: the joint filters' part of the
+// work, slots: CTAs the device holds.
+constexpr int kJointCtas = 4;
+constexpr uint64_t kJointMin = 4096;  // smaller filters stay on one CTA
+int pf_batched_joint_launch(const BatchedArgs &a, const int *order, int nj, int nf, double share, int threads,
+    int slots, int *queue, cudaStream_t s);
 
 }  // namespace mckl_b200

@@ -540,6 +540,59 @@ struct FilterScalars {
     int flat;
 };
 
+// ---- a filter run by a cluster of CTAs (FilterRun::joint_step) --------------
+// What the CTAs of a cluster tell one another: up to three words per slot, two
+// sets in turn (a CTA that writes set n + 2 is behind the barrier of n + 1, which
+// every CTA reaches only after it has read set n).
+// Working memory of a cluster, per unit of its filter (and one entry more for an
+// odd last particle).
+struct JointTerms {
+    float4 *e;   // [2 u, 2 u + 1]: the unit's log-weights, then its terms (unused slots -inf, then 0)
+    double *sc;  // [u]: the factor that takes the sums to the unit's running maximum
+};
+
+struct JointShared {
+    unsigned long long xs[2][3][32];
+    uint32_t ebase[9];  // empty slots before each CTA's particles
+    int f;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_sync()
+{
+    cluster_arrive();
+    cluster_wait();
+}
+
+// Store v in *p of CTA `rank`'s shared memory.
+template <typename T>
+__device__ __forceinline__ void cluster_store(T *p, uint32_t rank, T v)
+{
+    uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    if constexpr (sizeof(T) == 8) {
+        asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(r), "l"(static_cast<unsigned long long>(v)) : "memory");
+    } else {
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(r), "r"(static_cast<uint32_t>(v)) : "memory");
+    }
+}
+
 // One filter run by one CTA: state, and the step of the particle filter.
 //
 // SHADOW: every particle also carries an FP64 copy, propagated with the same
@@ -926,6 +979,384 @@ struct FilterRun {
         Ls_prev = L_prev;
         return true;
     }
+
+    // The grid points (U + i) / N at or below c 2^-62 (the comment in step()).
+    struct GridCount {
+        uint32_t N32;
+        uint64_t ulo;
+        int64_t uhi;
+        __device__ __forceinline__ uint32_t operator()(uint64_t c) const
+        {
+            const uint64_t a = static_cast<uint64_t>(N32) * static_cast<uint32_t>(c);
+            const uint64_t m = static_cast<uint64_t>(N32) * static_cast<uint32_t>(c >> 32) + (a >> 32);
+            const uint64_t xlo = ((m << 32) | static_cast<uint32_t>(a)) << 2;
+            const int64_t dhi = static_cast<int64_t>(m >> 30) - uhi - (xlo < ulo ? 1 : 0);
+            return dhi < 0 ? 0u : (dhi + 1 >= static_cast<int64_t>(N32) ? N32 : static_cast<uint32_t>(dhi) + 1u);
+        }
+    };
+
+    // step() by the CLUSTER CTAs of a cluster (rank cr), with the same bits.
+    //
+    // A large filter on one CTA is the tail of the whole batch: 65536 particles
+    // take ~440 us a step there, whatever the other SMs do.  What step() computes
+    // depends on which thread meets which unit in which order -- the
+    // normaliser's terms are rounded in FP32 relative to the thread's running
+    // maximum -- so the cluster keeps step()'s THREADS threads as virtual ones
+    // and splits their work: CTA cr owns virtual warps cr NW / CLUSTER .., and
+    // its warps take the units of a virtual warp in CLUSTER consecutive
+    // segments.
+    //   A  moves and weighs the segment's units and keeps their log-weights;
+    //   B  with the maxima of the segments before: the running maximum, hence
+    //      the units' terms and the factors between maxima;
+    //   C  one thread per virtual thread adds its terms in order, in FP64;
+    // the sums then meet in step()'s own tree.  The resampling splits the
+    // particles into CLUSTER ranges of tiles: the fixed-point totals of the
+    // ranges and their empty slots are exact, so their prefixes are too.
+    template <int CLUSTER, bool STAGEX>
+    __device__ bool joint_step(int t, double yt_d, uint32_t cr, const JointTerms &jt, JointShared *js, uint32_t &set,
+        R *shr, unsigned long long *shu, uint32_t *shj, R *shx)
+    {
+        static_assert(!SHADOW && sizeof(R) == 4, "FP32 terms");
+        constexpr int NW = THREADS / 32, VW = NW / CLUSTER;  // virtual warps per CTA
+        static_assert(NW % CLUSTER == 0, "whole virtual warps per CTA");
+        using O = Math<R>;
+        const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const uint32_t vwl = warp / CLUSTER, seg = warp % CLUSTER;
+        const uint32_t vt = (cr * VW + vwl) * 32 + lane;
+        const uint64_t N = lay.N;
+        const uint32_t N32 = static_cast<uint32_t>(N), units = static_cast<uint32_t>(lay.units);
+        const uint32_t fullu = static_cast<uint32_t>(lay.m * NoiseLayout::kUnits);
+        const uint32_t K = (units + THREADS - 1) / THREADS, KS = (K + CLUSTER - 1) / CLUSTER;
+        const uint32_t u0 = vt + seg * KS * THREADS;
+        const uint32_t uend = min(units, min(K, (seg + 1) * KS) * THREADS);
+        const bool odd = (N & 1) && vt == THREADS - 1 && seg == CLUSTER - 1;  // this thread moves the last particle
+        st.x = xc;
+        st.init = (t == 0);
+        st.yt_d = yt_d;
+        st.yt = static_cast<R>(yt_d);
+        // ---- A
+        R ms = -INFINITY;
+        for (uint32_t u = u0; u < uend; u += THREADS) {
+            R v[8];
+            double vs[8];
+            int lo, hi;
+            uint32_t wr[4], wa[4], pa[4], pb[4];
+            uint64_t src;
+            typename Step<R, SHADOW, Model>::Old old;
+            lay.slots(t, u, pa, pb, &lo, &hi, &src);
+            if (!st.init && u + THREADS < uend && u + THREADS < fullu) {
+                const uint32_t un = u + THREADS, c = un / 129u, pn = c * 1024u + 4u * (un - c * 129u);
+                prefetch_l1(st.x + pn);
+                prefetch_l1(st.x + pn + 512);
+                if (!st.flat) {
+                    prefetch_l1(st.l + pn);
+                    prefetch_l1(st.l + pn + 512);
+                }
+            }
+            lay.words(gm, u, src, wr, wa);
+            st.load4(pa, pb, lo, hi, old);
+            st.move4(wr, wa, pa, pb, lo, hi, old, v, vs);
+            if (t > 0) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (!(k >= 2 * lo && k < 2 * hi)) v[k] = -INFINITY;
+                    ms = fmax(ms, v[k]);
+                }
+                jt.e[2 * u] = make_float4(v[0], v[1], v[2], v[3]);
+                jt.e[2 * u + 1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+        R vodd = 0;
+        if (odd) {
+            uint32_t w0, w1;
+            lay.odd_words(gm, t, &w0, &w1);
+            st.one(O::mul(O::radius(u01oc<R>(w0)), O::cos2pi(u01oc<R>(w1))), N - 1, vodd);
+            if (t > 0) ms = fmax(ms, vodd);
+        }
+        if (t == 0) {
+            cluster_sync();
+            return false;
+        }
+        // the segments' maxima within the CTA, the CTA's to the cluster
+        R *segm = reinterpret_cast<R *>(shj);  // [vwl][seg][lane]
+        segm[threadIdx.x] = ms;
+        const R cm = block_max(ms, shr);
+        set ^= 1;
+        if (threadIdx.x < CLUSTER)
+            cluster_store(&js->xs[set][0][cr], threadIdx.x, static_cast<unsigned long long>(__float_as_uint(cm)));
+        __syncwarp();
+        cluster_arrive();  // the wait is behind B and C's chain
+        // ---- B
+        R m = -INFINITY;
+        for (uint32_t q = 0; q < seg; ++q) m = fmax(m, segm[(vwl * CLUSTER + q) * 32 + lane]);
+        // Lse::add's step to a new running maximum: the factor of the sums so far
+        auto meet = [&m](R g) {
+            double sc = 1.0;
+            if (g > m) {
+                sc = (m == -INFINITY) ? 0.0 : ::exp(static_cast<double>(m) - static_cast<double>(g));
+                m = g;
+            }
+            return sc;
+        };
+        for (uint32_t u = u0; u < uend; u += THREADS) {
+            const float4 a = jt.e[2 * u], b = jt.e[2 * u + 1];
+            jt.sc[u] = meet(fmax(fmax(fmax(a.x, a.y), fmax(a.z, a.w)), fmax(fmax(b.x, b.y), fmax(b.z, b.w))));
+            const auto ex = [m](R v) { return v == -INFINITY ? R(0) : O::exp(O::sub(v, m)); };
+            jt.e[2 * u] = make_float4(ex(a.x), ex(a.y), ex(a.z), ex(a.w));
+            jt.e[2 * u + 1] = make_float4(ex(b.x), ex(b.y), ex(b.z), ex(b.w));
+        }
+        if (odd) {
+            jt.sc[units] = meet(vodd);
+            jt.e[2 * units] = make_float4(O::exp(O::sub(vodd, m)), 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        // ---- C
+        double as = 0.0, aq = 0.0;
+        if (seg == 0) {
+            auto factor = [&as, &aq](double sc) {
+                as = __dmul_rn(as, sc);
+                aq = __dmul_rn(aq, __dmul_rn(sc, sc));
+            };
+            auto term = [&as, &aq](R ef) {  // a zero adds nothing
+                const double e = static_cast<double>(ef);
+                as = __dadd_rn(as, e);
+                aq = __fma_rn(e, e, aq);
+            };
+            // the next unit's words are read ahead of this one's chain
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            double f = 1.0;
+            if (vt < units) {
+                a = jt.e[2 * vt];
+                b = jt.e[2 * vt + 1];
+                f = jt.sc[vt];
+            }
+            for (uint32_t u = vt; u < units; u += THREADS) {
+                const uint32_t un = u + THREADS < units ? u + THREADS : u;
+                const float4 an = jt.e[2 * un], bn = jt.e[2 * un + 1];
+                const double fn = jt.sc[un];
+                factor(f);
+                term(a.x); term(a.y); term(a.z); term(a.w);
+                term(b.x); term(b.y); term(b.z); term(b.w);
+                a = an;
+                b = bn;
+                f = fn;
+            }
+            if ((N & 1) && vt == THREADS - 1) {
+                factor(jt.sc[units]);
+                term(jt.e[2 * units].x);
+            }
+        }
+        __syncwarp();
+        cluster_wait();
+        R M = -INFINITY;
+#pragma unroll
+        for (int q = 0; q < CLUSTER; ++q) M = fmax(M, __uint_as_float(static_cast<uint32_t>(js->xs[set][0][q])));
+        set ^= 1;
+        if (seg == 0) {
+            R mv = -INFINITY;  // the virtual thread's maximum
+            for (uint32_t q = 0; q < CLUSTER; ++q) mv = fmax(mv, segm[(vwl * CLUSTER + q) * 32 + lane]);
+            const double sc = (mv == -INFINITY) ? 0.0 : ::exp(static_cast<double>(mv) - static_cast<double>(M));
+            const double ws = warp_sum(__dmul_rn(as, sc)), wq = warp_sum(__dmul_rn(aq, __dmul_rn(sc, sc)));
+            if (lane < CLUSTER) {
+                cluster_store(&js->xs[set][0][cr * VW + vwl], lane,
+                    static_cast<unsigned long long>(__double_as_longlong(ws)));
+                cluster_store(&js->xs[set][1][cr * VW + vwl], lane,
+                    static_cast<unsigned long long>(__double_as_longlong(wq)));
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        const double S = warp_sum(lane < NW ? __longlong_as_double(static_cast<long long>(js->xs[set][0][lane])) : 0.0);
+        const double Q = warp_sum(lane < NW ? __longlong_as_double(static_cast<long long>(js->xs[set][1][lane])) : 0.0);
+        const double L = static_cast<double>(M) + log(S);
+        ll_sum += L - L_prev;
+        L_prev = log(S);
+        st.lshift = M;
+        st.flat = false;
+        const double ess = S * S / Q;
+        if (!(ess < static_cast<double>(N) * threshold)) return false;
+        // ---- systematic resampling (step()'s, by ranges of tiles)
+        ++events;
+        uint32_t wr[2];
+        {
+            WordCache wc{~0ull, {0, 0, 0, 0}};
+            const uint64_t a = 2 * (events - 1);
+            wr[0] = word_at(gr, a, wc);
+            wr[1] = word_at(gr, a + 1, wc);
+        }
+        const double U = __dadd_rn(__dmul_rn(static_cast<double>(wr[0]), 0x1p-64),
+            __dmul_rn(static_cast<double>(wr[1]), 0x1p-32));
+        const double invS62 = (1.0 / S) * 0x1p62;
+        constexpr int V = 8;
+        constexpr uint32_t TILE = THREADS * V;
+        const uint64_t U64 = U < 1.0 ? static_cast<uint64_t>(U * 0x1p64) : ~0ull;
+        const GridCount count{N32, U64 + 1, U64 == ~0ull ? 1 : 0};
+        const uint32_t span = ((N32 + TILE - 1) / TILE + CLUSTER - 1) / CLUSTER * TILE;  // particles per CTA
+        const uint32_t b0 = min(N32, cr * span), b1 = min(N32, b0 + span);
+        unsigned long long own = 0;
+        for (uint32_t q0 = b0 + threadIdx.x * V; q0 < b1; q0 += TILE) {
+            R lv[V];
+            if (q0 + V <= N32) {
+                ld8(st.l + q0, lv);
+            } else {
+#pragma unroll
+                for (int k = 0; k < V; ++k) lv[k] = q0 + k < N32 ? st.l[q0 + k] : R(-INFINITY);
+            }
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                own += __double2ull_rn(static_cast<double>(O::exp(O::sub(lv[k], M))) * invS62);
+        }
+        own = block_sum(own, shu);
+        set ^= 1;
+        if (threadIdx.x < CLUSTER) cluster_store(&js->xs[set][0][cr], threadIdx.x, own);
+        __syncwarp();
+        cluster_sync();
+        uint64_t carry = 0;
+        for (uint32_t q = 0; q < cr; ++q) carry += js->xs[set][0][q];
+        unsigned long long *shw64 = shu;
+        uint32_t *she = shj + THREADS + 1;
+        uint32_t ecarry = 0;  // empty slots of this range so far; they are listed from ep[b0]
+        for (uint32_t b = b0; b < b1; b += TILE) {
+            const uint32_t q0 = b + threadIdx.x * V;
+            const bool whole = q0 + V <= N32;
+            R lv[V];
+            if (whole) {
+                ld8(st.l + q0, lv);
+            } else {
+#pragma unroll
+                for (int k = 0; k < V; ++k) lv[k] = q0 + k < N32 ? st.l[q0 + k] : R(0);
+            }
+            unsigned long long C[V];
+            unsigned long long acc = 0;
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const double w62 = (whole || q0 + k < N32) ? static_cast<double>(O::exp(O::sub(lv[k], M))) * invS62 : 0.0;
+                acc += __double2ull_rn(w62);
+                C[k] = acc;
+            }
+            unsigned long long tot;
+            const uint64_t base = carry + block_inclusive_sum_1b(acc, shw64, &tot) - acc;
+            carry += tot;
+            const uint32_t jm = count(base);
+            uint32_t j[V];
+#pragma unroll
+            for (int k = 0; k < V; ++k) j[k] = (q0 + k + 1 >= N32) ? N32 : count(base + C[k]);
+            uint32_t ne = 0;
+#pragma unroll
+            for (int k = 0; k < V; ++k) ne += (q0 + k < N32 && j[k] == (k == 0 ? jm : j[k - 1])) ? 1u : 0u;
+            uint32_t etot;
+            uint32_t En = ecarry + block_inclusive_sum_1b(ne, she, &etot) - ne;
+            ecarry += etot;
+            uint32_t sv[V];
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const uint32_t p = q0 + k, jb = k == 0 ? jm : j[k - 1];
+                sv[k] = jb + En - p;  // less the empty slots of the ranges before
+                if ((whole || p < N32) && j[k] == jb) ep[b0 + En++] = p;
+            }
+            if (whole) {
+                st8(sS + q0, sv);
+            } else {
+#pragma unroll
+                for (int k = 0; k < V; ++k)
+                    if (q0 + k < N32) sS[q0 + k] = sv[k];
+            }
+        }
+        set ^= 1;
+        if (threadIdx.x < CLUSTER)
+            cluster_store(&js->xs[set][0][cr], threadIdx.x, static_cast<unsigned long long>(ecarry));
+        __syncwarp();
+        cluster_sync();
+        if (threadIdx.x <= CLUSTER) {
+            uint32_t e = 0;
+            for (uint32_t q = 0; q < threadIdx.x; ++q) e += static_cast<uint32_t>(js->xs[set][0][q]);
+            js->ebase[threadIdx.x] = e;
+        }
+        // ---- placement of this range's parents
+        uint32_t *nbig = shj + THREADS + 34, *big = nbig + 1;
+        if (threadIdx.x == 0) *nbig = 0;
+        __syncthreads();
+        const uint32_t ne = js->ebase[CLUSTER], eb = js->ebase[cr];
+        n_empty = ne;
+        // the e-th empty slot of the filter; ec: a range at or before its own
+        auto slot_of = [&](uint32_t e) {
+            uint32_t q = cr;
+            while (e < js->ebase[q]) --q;
+            while (e >= js->ebase[q + 1]) ++q;
+            return ep[q * span + (e - js->ebase[q])];
+        };
+        // prefix of particle p, the first of a range or inside this one
+        auto prefix = [&](uint32_t p) { return p >= N32 ? ne : sS[p] + (p < b1 ? eb : js->ebase[cr + 1]); };
+        uint32_t *wsw = shj + ws_offset<THREADS>() + warp * kWs;
+        R *wx = STAGEX ? shx + warp * kWarpParents : nullptr;
+        for (uint32_t b = b0; b < b1; b += TILE) {
+            const uint32_t P0 = b + warp * kWarpParents;
+            if (P0 >= b1) continue;  // warp-uniform; the loop holds no CTA barrier
+            const uint32_t q0 = P0 + lane * V;
+            {
+                uint32_t ss[V];
+                R xv[V];
+                if (q0 + V <= N32) {
+                    ld8(sS + q0, ss);
+                    if constexpr (STAGEX) ld8(xc + q0, xv);
+#pragma unroll
+                    for (int k = 0; k < V; ++k) ss[k] += eb;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < V; ++k) {
+                        ss[k] = q0 + k < N32 ? sS[q0 + k] + eb : ne;
+                        if constexpr (STAGEX) xv[k] = q0 + k < N32 ? xc[q0 + k] : R(0);
+                    }
+                }
+                st8(wsw + lane * V, ss);
+                if constexpr (STAGEX) st8(wx + lane * V, xv);
+            }
+            if (lane == 31) wsw[kWarpParents] = prefix(q0 + V);
+            __syncwarp();
+            const uint32_t A = wsw[0], B = wsw[kWarpParents];
+            uint32_t queued = 0;
+            if (B - A > kWarpCopies && lane == 0) {
+                const uint32_t q = atomicAdd(nbig, 1u);
+                if (q < kBigParents) {
+                    big[q] = P0;
+                    queued = 1;
+                }
+            }
+            queued = __shfl_sync(0xffffffffu, queued, 0);
+            if (!queued) {
+                for (uint32_t e = A + lane; e < B; e += 32) {
+                    uint32_t lo = 0;
+#pragma unroll
+                    for (uint32_t h = kWarpParents / 2; h >= 1; h >>= 1) lo += wsw[lo + h] <= e ? h : 0;
+                    const uint32_t slot = slot_of(e);
+                    xc[slot] = STAGEX ? wx[lo] : xc[P0 + lo];
+                }
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        const uint32_t nb = min(*nbig, kBigParents);
+        uint32_t *wsc = shj + ws_offset<THREADS>();
+        for (uint32_t i = 0; i < nb; ++i) {
+            const uint32_t P0 = big[i];
+            for (uint32_t k = threadIdx.x; k <= kWarpParents; k += THREADS)
+                wsc[k] = P0 + k < b1 ? sS[P0 + k] + eb : prefix(min(P0 + k, b1));
+            __syncthreads();
+            const uint32_t A = wsc[0], B = wsc[kWarpParents];
+            for (uint32_t e = A + threadIdx.x; e < B; e += THREADS) {
+                uint32_t lo = 0;
+#pragma unroll
+                for (uint32_t h = kWarpParents / 2; h >= 1; h >>= 1) lo += wsc[lo + h] <= e ? h : 0;
+                const uint32_t slot = slot_of(e);
+                xc[slot] = xc[P0 + lo];
+            }
+            __syncthreads();
+        }
+        cluster_sync();
+        st.flat = true;
+        L_prev = log(static_cast<double>(N));
+        return true;
+    }
 };
 
 // `par` (nullable): the filters' model parameters, which the shadow run
@@ -973,6 +1404,78 @@ __global__ void __launch_bounds__(THREADS, MINB) k_pf_batched(const BatchedFilte
     }
 }
 
+
+// k_pf_batched for a batch whose largest filters would be its tail: a grid of
+// clusters.  The first nj filters of the order (the largest) are run by a
+// cluster each, pulled from queue[1]; the others by a CTA each, from queue[0], as
+// k_pf_batched does.  The first ncj clusters start with the joint filters, the
+// rest with the others (the largest of those would be the tail if they had to
+// wait), and each goes on to the other kind when its own is done.  terms:
+// JointTerms of terms_units units (even; the most of any filter, and one more)
+// for each of the first nct clusters, which alone take joint filters.
+template <typename R, int THREADS, int MINB, int CLUSTER>
+__global__ void __launch_bounds__(THREADS, MINB) k_pf_batched_joint(const BatchedFilter *filt, const int *order, int nj,
+    int nf, int ncj, int nct, const double *y, int T, double threshold, R *xa, R *lw, uint32_t *scanS, uint32_t *epos,
+    double *loglik, uint32_t *nresampled, int *queue, char *terms, uint64_t terms_units)
+{
+    __shared__ double shd[33];
+    __shared__ R shr[33];
+    __shared__ unsigned long long shu[33];
+    __shared__ __align__(16) uint32_t shj[shj_words<THREADS>()];
+    constexpr bool kStageX = THREADS <= 512 && sizeof(R) * (THREADS / 32) * kWarpParents <= 16384;
+    __shared__ __align__(16) R shx[kStageX ? (THREADS / 32) * kWarpParents : 1];
+    __shared__ JointShared js;
+    __shared__ int sh_f;
+    const uint32_t cr = cluster_rank();
+    const int cluster = static_cast<int>(blockIdx.x / CLUSTER);
+    uint32_t set = 0;
+    char *tb = terms + static_cast<uint64_t>(cluster) * terms_units * (2 * sizeof(float4) + sizeof(double));
+    const JointTerms jt{reinterpret_cast<float4 *>(tb), reinterpret_cast<double *>(tb + terms_units * 2 * sizeof(float4))};
+    for (int pass = 0; pass < 2; ++pass) {
+        if ((pass == 0) == (cluster < ncj)) {
+            while (cluster < nct) {
+                cluster_sync();  // every CTA runs, and is done with the last filter
+                if (cr == 0 && threadIdx.x == 0) {
+                    const int k = atomicAdd(queue + 1, 1);
+                    const int f = k < nj ? order[k] : -1;
+                    for (uint32_t q = 0; q < CLUSTER; ++q) cluster_store(&js.f, q, f);
+                }
+                __syncwarp();
+                cluster_sync();
+                const int f = js.f;
+                if (f < 0) break;
+                FilterRun<R, THREADS, false> run;
+                run.setup(filt[f], xa, nullptr, lw, scanS, epos, nullptr, nullptr, nullptr, threshold);
+                const double *yf = y + static_cast<uint64_t>(f) * (T + 1);
+                for (int t = 0; t <= T; ++t)
+                    run.template joint_step<CLUSTER, kStageX>(t, yf[t], cr, jt, &js, set, shr, shu, shj, shx);
+                if (cr == 0 && threadIdx.x == 0) {
+                    loglik[f] = run.ll_sum;
+                    nresampled[f] = static_cast<uint32_t>(run.events);
+                }
+            }
+        } else {
+            while (true) {
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    const int k = nj + atomicAdd(queue, 1);
+                    sh_f = k < nf ? order[k] : -1;
+                }
+                __syncthreads();
+                const int f = sh_f;
+                if (f < 0) break;
+                FilterRun<R, THREADS, false> run;
+                run.setup(filt[f], xa, nullptr, lw, scanS, epos, nullptr, nullptr, nullptr, threshold);
+                const double *yf = y + static_cast<uint64_t>(f) * (T + 1);
+                for (int t = 0; t <= T; ++t) run.template step<kStageX>(t, yf[t], shd, shr, shu, shj, shx);
+                if (threadIdx.x == 0) {
+                    loglik[f] = run.ll_sum;
+                    nresampled[f] = static_cast<uint32_t>(run.events);
+                }
+            }
+        }
+    }
+}
 
 }  // namespace batched_detail
 }  // namespace mckl_b200
