@@ -24,26 +24,26 @@ __device__ __forceinline__ Ctx make_ctx(Shared &sh, const Global &g, unsigned T)
 }
 
 // A tile's dynamic shared memory: its values and its 64-bit integers, padded.
-template <int PER>
+template <int TILE>
 struct TileMem {
-    double v[padded(kThreads * PER)];
-    long long q[padded(kThreads * PER)];
+    double v[padded(TILE)];
+    long long q[padded(TILE)];
 };
 
-template <int PER, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_coop_weight(Global g, unsigned T, uint64_t N, double *W,
+template <int THR, int PER>
+__global__ void __launch_bounds__(THR, 1) k_coop_weight(Global g, unsigned T, uint64_t N, double *W,
     const double *v, int add_log, CoopResult *out)
 {
     extern __shared__ __align__(16) unsigned char coop_dyn[];
     __shared__ Shared sh;
-    TileMem<PER> &tm = *reinterpret_cast<TileMem<PER> *>(coop_dyn);
+    TileMem<THR * PER> &tm = *reinterpret_cast<TileMem<THR * PER> *>(coop_dyn);
     Ctx c = make_ctx(sh, g, T);
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE;
     double m = -__longlong_as_double(0x7ff0000000000000ll);
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         if (base + o < N) {
             const double lw = add_log ? __dadd_rn(dd::log(W[base + o]), v[base + o]) : v[base + o];
             tm.v[pad(o)] = lw;
@@ -52,11 +52,11 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_weight(Global g, unsign
     }
     WeightOut r;
     Approx ap;
-    if (!weight_phase<PER>(c, tm.v, tm.q, N, m, r, ap)) return;
+    if (!weight_phase<THR, PER>(c, tm.v, tm.q, N, m, r, ap)) return;
     const double inv = __ddiv_rn(1.0, r.accw);
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         if (base + o < N) W[base + o] = __dmul_rn(inv, tm.v[pad(o)]);
     }
     if (c.tile == 0 && threadIdx.x == 0) {
@@ -67,52 +67,52 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_weight(Global g, unsign
     }
 }
 
-template <int PER, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_coop_resample(Global g, unsigned T, int scheme, uint64_t N,
+template <int THR, int PER>
+__global__ void __launch_bounds__(THR, 1) k_coop_resample(Global g, unsigned T, int scheme, uint64_t N,
     uint64_t M, const double *W, const double *canon, double *ubuf, uint64_t *rep, CoopResult *out)
 {
     extern __shared__ __align__(16) unsigned char coop_dyn[];
     __shared__ Shared sh;
-    TileMem<PER> &tm = *reinterpret_cast<TileMem<PER> *>(coop_dyn);
+    TileMem<THR * PER> &tm = *reinterpret_cast<TileMem<THR * PER> *>(coop_dyn);
     Ctx c = make_ctx(sh, g, T);
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE;
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         tm.v[pad(o)] = base + o < N ? W[base + o] : 0.0;
     }
     __syncthreads();
     uint64_t R;
-    if (!resample_phase<PER>(c, tm.v, tm.q, N, M, scheme, [canon](uint64_t j) { return __ldg(canon + j); },
+    if (!resample_phase<THR, PER>(c, tm.v, tm.q, N, M, scheme, [canon](uint64_t j) { return __ldg(canon + j); },
             [W](uint64_t i) { return W[i]; }, ubuf, nullptr, &R, nullptr))
         return;
     __syncthreads();
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         if (base + o < N) rep[base + o] = static_cast<uint64_t>(tm.q[pad(o)]);
     }
     if (c.tile == 0 && threadIdx.x == 0) out->used = R;
 }
 
-template <int PER, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_coop_index(Global g, unsigned T, uint64_t N, uint64_t M,
+template <int THR, int PER>
+__global__ void __launch_bounds__(THR, 1) k_coop_index(Global g, unsigned T, uint64_t N, uint64_t M,
     const uint64_t *rep, uint32_t *surp, uint64_t *idx)
 {
     extern __shared__ __align__(16) unsigned char coop_dyn[];
     __shared__ Shared sh;
-    TileMem<PER> &tm = *reinterpret_cast<TileMem<PER> *>(coop_dyn);
+    TileMem<THR * PER> &tm = *reinterpret_cast<TileMem<THR * PER> *>(coop_dyn);
     Ctx c = make_ctx(sh, g, T);
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE;
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         tm.q[pad(o)] = base + o < N ? static_cast<long long>(rep[base + o]) : 0;
     }
     __syncthreads();
-    index_phase<PER>(c, tm.v, tm.q, N, M, surp, [idx](uint64_t d) { idx[d] = d; },
+    index_phase<THR, PER>(c, tm.v, tm.q, N, M, surp, [idx](uint64_t d) { idx[d] = d; },
         [idx](uint64_t d, uint64_t p) { idx[d] = p; });
 }
 
@@ -163,11 +163,11 @@ __device__ __forceinline__ void sincos_rn(double x, double *s, double *c)
 // The Normal(0, sd) draws of step t for the tile's particles, normal_distribution's
 // layout and arithmetic (rng.cu: k_normal, k_normal_odd), each handed to
 // put(local particle, value).  The tile's words are staged in shared memory.
-template <int PER, class Put>
+template <int THR, int PER, class Put>
 __device__ __forceinline__ void tile_normals(Ctx &c, const PhiloxGen &g, uint64_t N, uint64_t t, double sd,
     const Put &put)
 {
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE;
     if (base >= N) return;
     const uint32_t len = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), N - base));
@@ -175,7 +175,7 @@ __device__ __forceinline__ void tile_normals(Ctx &c, const PhiloxGen &g, uint64_
     const uint64_t a0 = t * (N + 2 * (N & 1)) + base, b0 = a0 >> 2;
     const uint32_t s0 = static_cast<uint32_t>(a0 & 3), nb = (s0 + len + (odd ? 2 : 0) + 3) >> 2;
     __syncthreads();  // the words share their memory with the windows
-    for (uint32_t i = threadIdx.x; i < nb; i += kThreads) {
+    for (uint32_t i = threadIdx.x; i < nb; i += THR) {
         uint32_t blk[4];
         g.block(Ctr{{b0 + i + 1, 0, 0, 0}}, blk);
         c.sh->words[i] = make_uint4(blk[0], blk[1], blk[2], blk[3]);
@@ -184,7 +184,7 @@ __device__ __forceinline__ void tile_normals(Ctx &c, const PhiloxGen &g, uint64_
     const uint32_t *w = reinterpret_cast<const uint32_t *>(c.sh->words) + s0;
     const uint32_t full = len & ~1023u, nu = (len - full) / 2;  // pairs of the partial chunk
 #pragma unroll 2
-    for (uint32_t p = threadIdx.x; p < TILE / 2; p += kThreads) {
+    for (uint32_t p = threadIdx.x; p < TILE / 2; p += THR) {
         const uint32_t cb = (p >> 9) * 1024, i = p & 511;
         const uint32_t half = cb < full ? 512 : nu;
         if (cb > full || (cb == full && i >= nu)) continue;
@@ -195,7 +195,7 @@ __device__ __forceinline__ void tile_normals(Ctx &c, const PhiloxGen &g, uint64_
         put(cb + i, __dmul_rn(r, sn));
         put(cb + half + i, __dmul_rn(r, cs));
     }
-    if (odd && threadIdx.x == kThreads - 1) {
+    if (odd && threadIdx.x == THR - 1) {
         const double r = __dmul_rn(sd, __dsqrt_rn(__dmul_rn(-2.0, log_rn(u01_f64(kOC, w[len])))));
         double sn, cs;
         sincos_rn(__dmul_rn(RealOps<double>::kTwoPi, u01_f64(kOC, w[len + 1])), &sn, &cs);
@@ -203,14 +203,14 @@ __device__ __forceinline__ void tile_normals(Ctx &c, const PhiloxGen &g, uint64_
     }
 }
 
-template <int PER, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsigned T, FilterArgs a)
+template <int THR, int PER>
+__global__ void __launch_bounds__(THR, 1) k_coop_filter(Global g, unsigned T, FilterArgs a)
 {
     extern __shared__ __align__(16) unsigned char coop_dyn[];
     __shared__ Shared sh;
-    TileMem<PER> &tm = *reinterpret_cast<TileMem<PER> *>(coop_dyn);
+    TileMem<THR * PER> &tm = *reinterpret_cast<TileMem<THR * PER> *>(coop_dyn);
     Ctx c = make_ctx(sh, g, T);
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     const uint64_t N = a.N, base = static_cast<uint64_t>(c.tile) * TILE;
     const PhiloxGen gm{a.mkey[0], a.mkey[1]}, gr{a.rkey[0], a.rkey[1]};
     const bool lead = c.tile == 0 && threadIdx.x == 0;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
     int cur = 0;
     double *x = a.xb[0];
     Approx ap;           // of the step's terms
-    tile_normals<PER>(c, gm, N, 0, a.sd0, [&](uint32_t o, double e) { x[base + o] = e; });
+    tile_normals<THR, PER>(c, gm, N, 0, a.sd0, [&](uint32_t o, double e) { x[base + o] = e; });
     __syncthreads();
     for (uint64_t t = 0; t <= a.T; ++t) {
         if (t > 0) {
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
             double m = -__longlong_as_double(0x7ff0000000000000ll);
             double *xn = a.xb[cur ^ 1];
             // the normalised weights are 1 / accw times the terms kept in tm.v
-            tile_normals<PER>(c, gm, N, t, 1.0, [&](uint32_t o, double e) {
+            tile_normals<THR, PER>(c, gm, N, t, 1.0, [&](uint32_t o, double e) {
                 const double v = __dadd_rn(__dmul_rn(a.phi, x[base + o]), __dmul_rn(a.sx, e));
                 xn[base + o] = v;
                 const double r = __dsub_rn(yt, v);
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
             cur ^= 1;
             x = xn;
             WeightOut r;
-            if (!weight_phase<PER>(c, tm.v, tm.q, N, m, r, ap)) return;
+            if (!weight_phase<THR, PER>(c, tm.v, tm.q, N, m, r, ap)) return;
             accw = r.accw;
             ess = r.ess;
             flat = false;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
         const Approx apw{__dmul_rn(inv, ap.A), __dmul_rn(inv, ap.own), __dmul_rn(inv, ap.M)};
         uint64_t R;
         const uint64_t rp = rpos;
-        if (!resample_phase<PER>(c, tm.v, tm.q, N, N, a.scheme,
+        if (!resample_phase<THR, PER>(c, tm.v, tm.q, N, N, a.scheme,
                 [&gr, rp](uint64_t j) {
                     const uint64_t w = rp + 2 * j;  // even: both words in one block
                     uint32_t blk[4];
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
         rpos += a.scheme % 3 == 2 ? 2 : 2 * R;
         __syncthreads();
         uint64_t *anc = a.anc ? a.anc + t * N : nullptr;
-        if (!index_phase<PER>(c, tm.v, tm.q, N, N, a.surp, [anc](uint64_t d) { if (anc) anc[d] = d; },
+        if (!index_phase<THR, PER>(c, tm.v, tm.q, N, N, a.surp, [anc](uint64_t d) { if (anc) anc[d] = d; },
                 [anc, x](uint64_t d, uint64_t p) {
                     if (anc) anc[d] = p;
                     x[d] = __ldcg(x + p);
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_coop_filter(Global g, unsign
     const double inv = __ddiv_rn(1.0, accw);
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         if (base + o < N) a.W[base + o] = flat ? a.equal : __dmul_rn(inv, tm.v[pad(o)]);
     }
     if (ties) atomicAdd(a.ties, ties);
@@ -314,7 +314,7 @@ constexpr size_t kSlotBytes = (2 * kMaxVals + 1) * kMaxTiles * sizeof(ulonglong2
 // CTAs of `kernel` that the current device holds at once (0 when it cannot
 // launch cooperatively); asked once per device.
 template <class K>
-int resident(K kernel, size_t dyn, std::atomic<int> *cache)
+int resident(K kernel, int threads, size_t dyn, std::atomic<int> *cache)
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 0;
@@ -325,7 +325,7 @@ int resident(K kernel, size_t dyn, std::atomic<int> *cache)
     cudaDeviceGetAttribute(&coopl, cudaDevAttrCooperativeLaunch, dev);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, dyn) != cudaSuccess || !coopl) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dyn) != cudaSuccess || !coopl) {
         cudaGetLastError();
         per_sm = 0;
     }
@@ -336,17 +336,18 @@ int resident(K kernel, size_t dyn, std::atomic<int> *cache)
 
 // The tiling of n elements (see smc_coop.cuh).
 struct Tiling {
-    int per;
+    int threads, per;
     unsigned T;
-    bool one_per_sm;
 };
 
 Tiling tiling(uint64_t n)
 {
-    const auto tiles = [n](uint64_t per) { return (n + kThreads * per - 1) / (kThreads * per); };
-    if (tiles(8) > kMaxTiles) return {0, 0, false};
-    if (tiles(2) <= 148) return {2, static_cast<unsigned>(tiles(2)), true};
-    return {8, static_cast<unsigned>(tiles(8)), tiles(8) <= 148};
+    static constexpr int kShapes[][2] = {{512, 2}, {1024, 4}, {1024, 7}, {1024, 8}};
+    for (const auto &k : kShapes) {
+        const uint64_t tile = static_cast<uint64_t>(k[0]) * k[1], T = (n + tile - 1) / tile;
+        if (T <= kMaxTiles) return {k[0], k[1], static_cast<unsigned>(T)};
+    }
+    return {0, 0, 0};
 }
 
 // Working memory of a launch of T tiles over n elements with `extra` more
@@ -376,12 +377,12 @@ int coop_scratch(const Tiling &t, uint64_t n, size_t extra, Global *g, CoopResul
 
 // Launch kernel instance K (T tiles) if the device holds it at once.
 template <class K, class... Args>
-int launch(K kernel, size_t dyn, std::atomic<int> *cache, unsigned T, cudaStream_t s, Args... args)
+int launch(K kernel, int threads, size_t dyn, std::atomic<int> *cache, unsigned T, cudaStream_t s, Args... args)
 {
-    if (static_cast<int>(T) > resident(kernel, dyn, cache)) return kCoopNo;
+    if (static_cast<int>(T) > resident(kernel, threads, dyn, cache)) return kCoopNo;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(T);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = dyn;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -406,14 +407,17 @@ int launch(K kernel, size_t dyn, std::atomic<int> *cache, unsigned T, cudaStream
     return MCKL_B200_OK;
 }
 
-#define COOP_LAUNCH(KERNEL, TILING, STREAM, ...)                                                    \
-    [&]() -> int {                                                                                             \
-        static std::atomic<int> cache_[3][16];                                                                 \
-        if ((TILING).per == 2)                                                                                 \
-            return launch(KERNEL<2, 1>, sizeof(TileMem<2>), cache_[0], (TILING).T, STREAM, __VA_ARGS__); \
-        if ((TILING).one_per_sm)                                                                               \
-            return launch(KERNEL<8, 1>, sizeof(TileMem<8>), cache_[1], (TILING).T, STREAM, __VA_ARGS__); \
-        return launch(KERNEL<8, 2>, sizeof(TileMem<8>), cache_[2], (TILING).T, STREAM, __VA_ARGS__); \
+#define COOP_SHAPE(KERNEL, THR, PER, SLOT, TILING, STREAM, ...) \
+    if ((TILING).threads == THR && (TILING).per == PER)         \
+        return launch(KERNEL<THR, PER>, THR, sizeof(TileMem<THR * PER>), cache_[SLOT], (TILING).T, STREAM, __VA_ARGS__);
+#define COOP_LAUNCH(KERNEL, TILING, STREAM, ...)                          \
+    [&]() -> int {                                                        \
+        static std::atomic<int> cache_[4][16];                            \
+        COOP_SHAPE(KERNEL, 512, 2, 0, TILING, STREAM, __VA_ARGS__)        \
+        COOP_SHAPE(KERNEL, 1024, 4, 1, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 7, 2, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 8, 3, TILING, STREAM, __VA_ARGS__)       \
+        return kCoopNo;                                                   \
     }()
 
 }  // namespace
@@ -455,7 +459,7 @@ int coop_rep_to_index(uint64_t N, uint64_t M, const uint64_t *rep, uint64_t *idx
     if (!t.T) return kCoopNo;
     Global g;
     char *more;
-    const int rc = coop_scratch(t, n, align256(static_cast<size_t>(t.T) * kThreads * t.per * sizeof(uint32_t)), &g, res, &more,
+    const int rc = coop_scratch(t, n, align256(static_cast<size_t>(t.T) * t.threads * t.per * sizeof(uint32_t)), &g, res, &more,
         s);
     if (rc != MCKL_B200_OK) return rc;
     if (t.T == 1) *res = nullptr;
@@ -469,7 +473,7 @@ int coop_filter(const CoopFilter &f, double *loglik, double *ess, uint8_t *resam
     if (!t.T) return kCoopNo;
     // results: loglik, ties, last, ess[T + 1], resampled[T + 1]
     const size_t rbytes = align256(24 + (T + 1) * 9);
-    const size_t tile_words = static_cast<size_t>(t.T) * kThreads * t.per;
+    const size_t tile_words = static_cast<size_t>(t.T) * t.threads * t.per;
     Global g;
     CoopResult *res;
     char *p;

@@ -18,11 +18,12 @@
 // loop over a thread's elements is rolled (with the loops unrolled and the
 // values in registers the weight call of 1001 particles took 56 us).
 //
-// Tiles: 512 threads of PER consecutive elements each.  PER = 2 for a cloud of
-// up to 1024 (one CTA) and where its tiles fit one per SM, since more CTAs
-// shorten every phase; PER = 8 for a cloud of one 4096-element tile (no
-// exchange at all) and for the largest clouds (two CTAs per SM).  Clouds of
-// more tiles than the chip holds CTAs take the multi-kernel step.
+// Tiles: THR threads of PER consecutive elements each, at most one tile per SM.
+// 512 x 2 while that many tiles of 1024 do (one CTA alone up to 1024 elements, a
+// cluster up to 8192), since more CTAs shorten every phase; then 1024 x 4, 7 or 8,
+// so that every SM has the same work (2^20 particles on 256 tiles of 4096, two
+// on most SMs: 97 us a filter step; on 147 tiles of 7168: 91 us).  Clouds of
+// more tiles than that take the multi-kernel step.
 #pragma once
 
 #include <cstdint>
@@ -37,8 +38,9 @@
 namespace mckl_b200 {
 namespace coop {
 
-constexpr int kThreads = 512, kWarps = kThreads / 32;
-constexpr unsigned kMaxTiles = 296;   // two CTAs on each of 148 SMs
+constexpr int kMaxWarps = 32;
+constexpr unsigned kMaxTiles = 148;   // one CTA per SM
+constexpr unsigned kMaxTile = 8192;   // elements
 constexpr unsigned kTileWin = 256;    // windows a tile can list
 constexpr unsigned kWin = 512;        // windows of a fold the walk takes
 constexpr unsigned kSegWin = 64;      // windows of one short fold (seg_fold)
@@ -62,7 +64,7 @@ struct Global {
 };
 
 struct Shared {
-    unsigned long long scr[2][2][kWarps];  // warp totals of the scans, alternating
+    unsigned long long scr[2][2][kMaxWarps];  // warp totals of the scans, alternating
     double tpre, tpmax, total;
     int elast, elast_all, ok;
     uint32_t pw[kMaxTiles + 1];            // windows (or empty slots) before each tile
@@ -72,19 +74,19 @@ struct Shared {
             int we[kWin];                  // the fold's windows in order
             double wx[kWin], wS[kWin];
             long long wP[kWin];
-            // short folds: up to four segments
-            int ge[4][kSegWin];
-            double gx[4][kSegWin];
-            long long gP[4][kSegWin];
+            // short folds: up to eight segments
+            int ge[8][kSegWin];
+            double gx[8][kSegWin];
+            long long gP[8][kSegWin];
         };
-        uint4 words[1028];                 // the filter's noise: a tile's Philox blocks
-        uint32_t empties[4096];            // a tile's empty slots in order
+        uint4 words[kMaxTile / 4 + 4];     // the filter's noise: a tile's Philox blocks
+        uint32_t empties[kMaxTile];        // a tile's empty slots in order
     };
     unsigned long long xs[2][kMaxVals][kMaxCluster];  // exchange slots of a cluster
-    long long gq[4];
-    unsigned gw[4];
-    int gel[4];
-    double gtot[4], dots[4];
+    long long gq[8];
+    unsigned gw[8];
+    int gel[8];
+    double gtot[8], dots[8];
 };
 
 struct Ctx {
@@ -209,6 +211,7 @@ __device__ __forceinline__ bool exchange(Ctx &c, unsigned long long (&v)[NV], bo
 
 // Exclusive sums (formed without a subtraction) and exclusive maxima of
 // nonnegative values, and the totals.
+template <int THR>
 __device__ __forceinline__ void scan_sum_max(Ctx &c, double v, double m, double &es, double &em, double &ts,
     double &tm)
 {
@@ -225,15 +228,15 @@ __device__ __forceinline__ void scan_sum_max(Ctx &c, double v, double m, double 
     double ps = __shfl_up_sync(0xffffffffu, is, 1), pm = __shfl_up_sync(0xffffffffu, im, 1);
     if (lane == 0) ps = pm = 0.0;
     c.flip ^= 1;
-    unsigned long long(*buf)[kWarps] = c.sh->scr[c.flip];
+    unsigned long long(*buf)[kMaxWarps] = c.sh->scr[c.flip];
     if (lane == 31) {
         buf[0][warp] = dbits(is);
         buf[1][warp] = dbits(im);
     }
     __syncthreads();
-    double ws = lane < kWarps ? bitsd(buf[0][lane]) : 0.0, wm = lane < kWarps ? bitsd(buf[1][lane]) : 0.0;
+    double ws = lane < THR / 32 ? bitsd(buf[0][lane]) : 0.0, wm = lane < THR / 32 ? bitsd(buf[1][lane]) : 0.0;
 #pragma unroll
-    for (int o = 1; o < kWarps; o <<= 1) {
+    for (int o = 1; o < THR / 32; o <<= 1) {
         const double us = __shfl_up_sync(0xffffffffu, ws, o), um = __shfl_up_sync(0xffffffffu, wm, o);
         if (lane >= o) {
             ws += us;
@@ -242,8 +245,8 @@ __device__ __forceinline__ void scan_sum_max(Ctx &c, double v, double m, double 
     }
     const double bs = __shfl_sync(0xffffffffu, ws, warp > 0 ? warp - 1 : 0);
     const double bm = __shfl_sync(0xffffffffu, wm, warp > 0 ? warp - 1 : 0);
-    ts = __shfl_sync(0xffffffffu, ws, kWarps - 1);
-    tm = __shfl_sync(0xffffffffu, wm, kWarps - 1);
+    ts = __shfl_sync(0xffffffffu, ws, THR / 32 - 1);
+    tm = __shfl_sync(0xffffffffu, wm, THR / 32 - 1);
     es = warp > 0 ? bs + ps : ps;
     em = warp > 0 ? fmax(bm, pm) : pm;
 }
@@ -260,6 +263,7 @@ __device__ __forceinline__ double warp_max_nonneg(double v)
 
 // Exclusive sums of nonnegative values (formed without a subtraction) and the
 // total; em: the maximum over the warps before this one, tm over all.
+template <int THR>
 __device__ __forceinline__ void scan_sum(Ctx &c, double v, double m, double &es, double &em, double &ts, double &tm)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -267,71 +271,74 @@ __device__ __forceinline__ void scan_sum(Ctx &c, double v, double m, double &es,
     double ps = __shfl_up_sync(0xffffffffu, is, 1);
     if (lane == 0) ps = 0.0;
     c.flip ^= 1;
-    unsigned long long(*buf)[kWarps] = c.sh->scr[c.flip];
+    unsigned long long(*buf)[kMaxWarps] = c.sh->scr[c.flip];
     if (lane == 31) {
         buf[0][warp] = dbits(is);
         buf[1][warp] = dbits(wmx);
     }
     __syncthreads();
-    double ws = lane < kWarps ? bitsd(buf[0][lane]) : 0.0;
-    const double wm = lane < kWarps ? bitsd(buf[1][lane]) : 0.0;
+    double ws = lane < THR / 32 ? bitsd(buf[0][lane]) : 0.0;
+    const double wm = lane < THR / 32 ? bitsd(buf[1][lane]) : 0.0;
 #pragma unroll
-    for (int o = 1; o < kWarps; o <<= 1) {
+    for (int o = 1; o < THR / 32; o <<= 1) {
         const double us = __shfl_up_sync(0xffffffffu, ws, o);
         if (lane >= o) ws += us;
     }
     const double bs = __shfl_sync(0xffffffffu, ws, warp > 0 ? warp - 1 : 0);
-    ts = __shfl_sync(0xffffffffu, ws, kWarps - 1);
+    ts = __shfl_sync(0xffffffffu, ws, THR / 32 - 1);
     tm = warp_max_nonneg(wm);
     em = warp_max_nonneg(lane < warp ? wm : 0.0);
     es = warp > 0 ? bs + ps : ps;
 }
 
 // Exclusive sums of two 64-bit integers, and the totals.
+template <int THR>
 __device__ __forceinline__ void scan_two(Ctx &c, long long a, long long b, long long &ea, long long &eb,
     long long &ta, long long &tb)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long ia = warp_inclusive_sum(a), ib = warp_inclusive_sum(b);
     c.flip ^= 1;
-    unsigned long long(*buf)[kWarps] = c.sh->scr[c.flip];
+    unsigned long long(*buf)[kMaxWarps] = c.sh->scr[c.flip];
     if (lane == 31) {
         buf[0][warp] = static_cast<unsigned long long>(ia);
         buf[1][warp] = static_cast<unsigned long long>(ib);
     }
     __syncthreads();
-    long long wa = lane < kWarps ? static_cast<long long>(buf[0][lane]) : 0;
-    long long wb = lane < kWarps ? static_cast<long long>(buf[1][lane]) : 0;
+    long long wa = lane < THR / 32 ? static_cast<long long>(buf[0][lane]) : 0;
+    long long wb = lane < THR / 32 ? static_cast<long long>(buf[1][lane]) : 0;
     wa = warp_inclusive_sum(wa);
     wb = warp_inclusive_sum(wb);
     const long long ba = __shfl_sync(0xffffffffu, wa, warp > 0 ? warp - 1 : 0);
     const long long bb = __shfl_sync(0xffffffffu, wb, warp > 0 ? warp - 1 : 0);
-    ta = __shfl_sync(0xffffffffu, wa, kWarps - 1);
-    tb = __shfl_sync(0xffffffffu, wb, kWarps - 1);
+    ta = __shfl_sync(0xffffffffu, wa, THR / 32 - 1);
+    tb = __shfl_sync(0xffffffffu, wb, THR / 32 - 1);
     ea = ia - a + (warp > 0 ? ba : 0);
     eb = ib - b + (warp > 0 ? bb : 0);
 }
 
+template <int THR>
 __device__ __forceinline__ double max_all(Ctx &c, double v)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = warp_max(v);
     c.flip ^= 1;
-    unsigned long long(*buf)[kWarps] = c.sh->scr[c.flip];
+    unsigned long long(*buf)[kMaxWarps] = c.sh->scr[c.flip];
     if (lane == 0) buf[0][warp] = dbits(v);
     __syncthreads();
-    return warp_max(bitsd(buf[0][lane & (kWarps - 1)]));
+    return warp_max(bitsd(buf[0][lane & (THR / 32 - 1)]));
 }
 
+template <int THR>
 __device__ __forceinline__ uint32_t min_all(Ctx &c, uint32_t v)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = __reduce_min_sync(0xffffffffu, v);
     c.flip ^= 1;
-    unsigned long long(*buf)[kWarps] = c.sh->scr[c.flip];
+    unsigned long long(*buf)[kMaxWarps] = c.sh->scr[c.flip];
     if (lane == 0) buf[0][warp] = v;
     __syncthreads();
-    return __reduce_min_sync(0xffffffffu, static_cast<uint32_t>(buf[0][lane & (kWarps - 1)]));
+    return __reduce_min_sync(0xffffffffu, static_cast<uint32_t>(buf[0][lane & (THR / 32 - 1)]));
 }
 
 // ---- the walk over a fold's windows (fold.cuh): the run before a window is
@@ -488,7 +495,7 @@ __device__ __forceinline__ void classify_tile(const Get &get, long long *s_q, ui
 // ---- the event-loop fold of one tile (fold.cuh), from the value s before it:
 // with PREFIX every partial sum replaces its value in s_v; returns the last.
 // len elements of the tile exist.
-template <int PER, bool PREFIX>
+template <int THR, int PER, bool PREFIX>
 __device__ __noinline__ double tile_exact(Ctx &c, double *s_v, long long *s_q, uint32_t len, double s)
 {
     constexpr uint32_t kStretch = 256;
@@ -531,7 +538,7 @@ __device__ __noinline__ double tile_exact(Ctx &c, double *s_v, long long *s_q, u
             own += q;
         }
         long long before, dummy, t0, t1;
-        scan_two(c, own, 0, before, dummy, t0, t1);
+        scan_two<THR>(c, own, 0, before, dummy, t0, t1);
         uint32_t first = 0xffffffffu;
         long long run = before;
 #pragma unroll 1
@@ -540,7 +547,7 @@ __device__ __noinline__ double tile_exact(Ctx &c, double *s_v, long long *s_q, u
             if (j0 + k >= cur && j0 + k < len && first == 0xffffffffu && (((ev >> k) & 1u) || K + run >= top))
                 first = j0 + k;
         }
-        const uint32_t cpos = min_all(c, first);
+        const uint32_t cpos = min_all<THR>(c, first);
         run = before;
 #pragma unroll 1
         for (int k = 0; k < PER; ++k) {
@@ -571,13 +578,13 @@ __device__ __noinline__ double tile_exact(Ctx &c, double *s_v, long long *s_q, u
 // predecessor's last value; with PREFIX the partial sums replace the values.
 // Taken when the windows do not fit their lists (ties everywhere) or a run left
 // its binade.
-template <int PER, bool PREFIX>
+template <int THR, int PER, bool PREFIX>
 __device__ __noinline__ bool fold_chain(Ctx &c, double *s_v, long long *s_q, uint64_t n, double *total,
     double *before)
 {
     ++c.chain_epoch;
-    const uint64_t base = static_cast<uint64_t>(c.tile) * (kThreads * PER);
-    const uint32_t len = base < n ? static_cast<uint32_t>(min(static_cast<uint64_t>(kThreads * PER), n - base)) : 0u;
+    const uint64_t base = static_cast<uint64_t>(c.tile) * (THR * PER);
+    const uint32_t len = base < n ? static_cast<uint32_t>(min(static_cast<uint64_t>(THR * PER), n - base)) : 0u;
     bool ok = true;
     if (threadIdx.x == 0) {
         unsigned long long b[1] = {0};
@@ -589,7 +596,7 @@ __device__ __noinline__ bool fold_chain(Ctx &c, double *s_v, long long *s_q, uin
     const double s_in = c.sh->tpre;
     __syncthreads();
     double s = s_in;
-    if (len) s = tile_exact<PER, PREFIX>(c, s_v, s_q, len, s_in);
+    if (len) s = tile_exact<THR, PER, PREFIX>(c, s_v, s_q, len, s_in);
     if (c.T > 1) {
         if (threadIdx.x == 0) {
             publish(c.g.chain + c.tile, dbits(s), c.chain_epoch);
@@ -617,7 +624,7 @@ struct Approx {
 };
 
 // The approximate sums of the values in s_v (0 past n).  False when a wait gave up.
-template <int PER>
+template <int THR, int PER>
 __device__ __forceinline__ bool fold_approx(Ctx &c, const double *s_v, Approx &ap)
 {
     double own = 0.0, mx = 0.0;
@@ -628,7 +635,7 @@ __device__ __forceinline__ bool fold_approx(Ctx &c, const double *s_v, Approx &a
         mx = fmax(mx, x);
     }
     double ex, em, ts, tm, tpre = 0.0, tpm = 0.0;
-    scan_sum(c, own, mx, ex, em, ts, tm);
+    scan_sum<THR>(c, own, mx, ex, em, ts, tm);
     if (c.T > 1) {
         unsigned long long x[2] = {dbits(ts), dbits(tm)};
         if (!exchange(c, x, false)) return false;
@@ -640,7 +647,7 @@ __device__ __forceinline__ bool fold_approx(Ctx &c, const double *s_v, Approx &a
             }
         } else {
             double e2, m2, t0, t1;
-            scan_sum_max(c, bitsd(x[0]), bitsd(x[1]), e2, m2, t0, t1);
+            scan_sum_max<THR>(c, bitsd(x[0]), bitsd(x[1]), e2, m2, t0, t1);
             if (threadIdx.x == c.tile) {
                 c.sh->tpre = e2;
                 c.sh->tpmax = m2;
@@ -662,12 +669,12 @@ __device__ __forceinline__ bool fold_approx(Ctx &c, const double *s_v, Approx &a
 // and the one before the thread's first element goes to *before.  What was
 // written to global memory before the call is visible after it (its exchange
 // carries data).  s_q is overwritten.  False when a wait gave up.
-template <int PER, bool PREFIX>
+template <int THR, int PER, bool PREFIX>
 __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint64_t n, const Approx ap,
     double *total, double *before)
 {
     Shared *sh = c.sh;
-    const uint64_t i0 = (static_cast<uint64_t>(c.tile) * kThreads + threadIdx.x) * PER;
+    const uint64_t i0 = (static_cast<uint64_t>(c.tile) * THR + threadIdx.x) * PER;
     if (threadIdx.x == 0) sh->elast = -1;
     __syncthreads();
     unsigned win;
@@ -675,7 +682,7 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
     classify_tile<PER>([s_v](int k) { return s_v[at<PER>(k)]; }, s_q, i0, n, c.T, ap.A, ap.own, ap.M, &win, &qs,
         &sh->elast);
     long long P, r, qtot, wtot;
-    scan_two(c, qs, __popc(win), P, r, qtot, wtot);
+    scan_two<THR>(c, qs, __popc(win), P, r, qtot, wtot);
     bool over = wtot > static_cast<long long>(c.T == 1 ? kWin : kTileWin);
     if (win && !over) {
         long long Pk = P;
@@ -728,19 +735,19 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
                 tw += w;
             }
         } else {
-            scan_two(c, static_cast<long long>(x[0]), wi, eq, ew, tq, tw);
+            scan_two<THR>(c, static_cast<long long>(x[0]), wi, eq, ew, tq, tw);
         }
         if (threadIdx.x < c.T) {
             sh->pq[threadIdx.x] = eq;
             sh->pw[threadIdx.x] = static_cast<uint32_t>(ew);
             // the tile that holds element n - 1 tells its run's binade
-            if (threadIdx.x == (n - 1) / (kThreads * PER)) sh->elast_all = el;
+            if (threadIdx.x == (n - 1) / (THR * PER)) sh->elast_all = el;
         }
         over = __syncthreads_or(wi > static_cast<long long>(kTileWin)) || tw > static_cast<long long>(kWin);
         W = static_cast<unsigned>(tw);
         Q = tq;
         if (!over) {
-            for (unsigned k = threadIdx.x; k < W; k += kThreads) {
+            for (unsigned k = threadIdx.x; k < W; k += THR) {
                 uint32_t lo = 0, hi = c.T;  // the last tile with pw <= k
                 while (hi - lo > 1) {
                     const uint32_t mid = (lo + hi) >> 1;
@@ -762,7 +769,7 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
         sh->ok = walk_windows(W, sh->wx, sh->wP, sh->we, sh->wS, Q, sh->elast_all, &sh->total) ? 1 : 0;
     __syncthreads();
     // `over` and the walk's outcome come from the same data in every CTA
-    if (over || !sh->ok) return fold_chain<PER, PREFIX>(c, s_v, s_q, n, total, before);
+    if (over || !sh->ok) return fold_chain<THR, PER, PREFIX>(c, s_v, s_q, n, total, before);
     *total = sh->total;
     if constexpr (PREFIX) {
         P += sh->pq[c.tile];
@@ -788,10 +795,10 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
 // fold of the segment's first `len` values get(k) (PER per thread, 0 beyond)
 // into sh->gtot[segment].  again(segment, j): value j, for a segment whose
 // windows do not fit their list.  s_q is overwritten.
-template <int PER, int SEGT, class Get, class Again>
+template <int THR, int PER, int SEGT, class Get, class Again>
 __device__ void seg_fold(Ctx &c, long long *s_q, uint32_t len, const Get &get, const Again &again)
 {
-    static_assert(kThreads / SEGT <= 4 && SEGT % 32 == 0, "segments");
+    static_assert(THR / SEGT <= 8 && SEGT % 32 == 0, "segments");
     constexpr int SW = SEGT / 32;  // warps per segment
     Shared *sh = c.sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seg = threadIdx.x / SEGT;
@@ -808,14 +815,14 @@ __device__ void seg_fold(Ctx &c, long long *s_q, uint32_t len, const Get &get, c
     double ps = __shfl_up_sync(0xffffffffu, is, 1);
     if (lane == 0) ps = 0.0;
     c.flip ^= 1;
-    unsigned long long(*buf)[kWarps] = sh->scr[c.flip];
+    unsigned long long(*buf)[kMaxWarps] = sh->scr[c.flip];
     if (lane == 31) {
         buf[0][warp] = dbits(is);
         buf[1][warp] = dbits(wmx);
     }
     __syncthreads();
-    double ws = lane < kWarps ? bitsd(buf[0][lane]) : 0.0;
-    const double wm = lane < kWarps ? bitsd(buf[1][lane]) : 0.0;
+    double ws = lane < THR / 32 ? bitsd(buf[0][lane]) : 0.0;
+    const double wm = lane < THR / 32 ? bitsd(buf[1][lane]) : 0.0;
 #pragma unroll
     for (int o = 1; o < SW; o <<= 1) {
         const double us = __shfl_up_sync(0xffffffffu, ws, o);
@@ -828,7 +835,12 @@ __device__ void seg_fold(Ctx &c, long long *s_q, uint32_t len, const Get &get, c
     const double ex = firstw ? ps : bs + ps;
     unsigned win;
     long long qs;
-    classify_tile<PER>(get, s_q, i0, len, 1, ex, own, em, &win, &qs, &sh->gel[seg]);
+    if (len == 0) {  // no segment here (the same for its whole warps)
+        win = 0;
+        qs = 0;
+    } else {
+        classify_tile<PER>(get, s_q, i0, len, 1, ex, own, em, &win, &qs, &sh->gel[seg]);
+    }
     const long long iq = warp_inclusive_sum(qs);
     const uint32_t iw = warp_inclusive_sum(static_cast<uint32_t>(__popc(win)));
     c.flip ^= 1;
@@ -838,8 +850,8 @@ __device__ void seg_fold(Ctx &c, long long *s_q, uint32_t len, const Get &get, c
         buf[1][warp] = iw;
     }
     __syncthreads();
-    long long wq = lane < kWarps ? static_cast<long long>(buf[0][lane]) : 0;
-    uint32_t ww = lane < kWarps ? static_cast<uint32_t>(buf[1][lane]) : 0;
+    long long wq = lane < THR / 32 ? static_cast<long long>(buf[0][lane]) : 0;
+    uint32_t ww = lane < THR / 32 ? static_cast<uint32_t>(buf[1][lane]) : 0;
 #pragma unroll
     for (int o = 1; o < SW; o <<= 1) {
         const long long uq = __shfl_up_sync(0xffffffffu, wq, o);
@@ -907,17 +919,17 @@ struct WeightOut {
     double ess, accw, lmax;
 };
 
-template <int PER>
+template <int THR, int PER>
 __device__ __forceinline__ bool weight_phase(Ctx &c, double *s_w, long long *s_q, uint64_t N, double m,
     WeightOut &out, Approx &ap)
 {
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE;
-    m = max_all(c, m);
+    m = max_all<THR>(c, m);
     if (c.T > 1) {
         unsigned long long x[1] = {static_cast<unsigned long long>(ordered_bits(m))};
         if (!exchange(c, x, false)) return false;
-        m = max_all(c, threadIdx.x < c.T ? from_ordered_bits(static_cast<long long>(x[0]))
+        m = max_all<THR>(c, threadIdx.x < c.T ? from_ordered_bits(static_cast<long long>(x[0]))
                                          : -__longlong_as_double(0x7ff0000000000000ll));
     }
     const double lmax = m;
@@ -927,17 +939,20 @@ __device__ __forceinline__ bool weight_phase(Ctx &c, double *s_w, long long *s_q
         const double e = in ? exp_rn(__dsub_rn(s_w[at<PER>(k)], lmax)) : 0.0;
         s_w[at<PER>(k)] = e;
     }
-    // the ESS's dot products: one short fold per chunk of 1024 particles
-    constexpr int SEGT = 1024 / PER, NSEG = kThreads / SEGT;
-    const uint64_t cb = base + static_cast<uint64_t>(threadIdx.x / SEGT) * 1024;
-    const uint32_t clen = cb < N ? static_cast<uint32_t>(min(static_cast<uint64_t>(1024), N - cb)) : 0u;
-    seg_fold<PER, SEGT>(c, s_q, clen,
+    // the ESS's dot products: one short fold per chunk of 1024 particles, by
+    // 128 threads of eight consecutive elements (all 512 of two for one chunk)
+    constexpr int NSEG = TILE / 1024, SP = NSEG == 1 ? 1024 / THR : 8, SEGT = 1024 / SP;
+    if constexpr (SP != PER) __syncthreads();
+    const int seg = threadIdx.x / SEGT;
+    const uint64_t cb = base + static_cast<uint64_t>(seg) * 1024;
+    const uint32_t clen = seg < NSEG && cb < N ? static_cast<uint32_t>(min(static_cast<uint64_t>(1024), N - cb)) : 0u;
+    seg_fold<THR, SP, SEGT>(c, s_q, clen,
         [s_w](int k) {
-            const double e = s_w[at<PER>(k)];
+            const double e = s_w[at<SP>(k)];
             return __dmul_rn(e, e);
         },
-        [s_w](int seg, uint32_t j) {
-            const double e = s_w[pad(seg * 1024 + j)];
+        [s_w](int sg, uint32_t j) {
+            const double e = s_w[pad(sg * 1024 + j)];
             return __dmul_rn(e, e);
         });
     const uint32_t nd = static_cast<uint32_t>((N + 1023) / 1024);
@@ -947,9 +962,9 @@ __device__ __forceinline__ bool weight_phase(Ctx &c, double *s_w, long long *s_q
         if (d < nd) dots[d] = c.sh->gtot[threadIdx.x];
     }
     double accw, before;
-    if (!fold_approx<PER>(c, s_w, ap) || !fold_grid<PER, false>(c, s_w, s_q, N, ap, &accw, &before)) return false;
-    constexpr int DP = (kMaxTiles * NSEG + kThreads - 1) / kThreads;
-    static_assert(DP <= PER, "the dots' increments fit the tile's");
+    if (!fold_approx<THR, PER>(c, s_w, ap) || !fold_grid<THR, PER, false>(c, s_w, s_q, N, ap, &accw, &before)) return false;
+    constexpr int DP = (kMaxTiles * NSEG + THR - 1) / THR;
+    static_assert(DP * THR <= TILE, "the dots' increments fit the tile's");
     if (c.T <= kMaxCluster) {  // a few
         if (threadIdx.x == 0) {
             double t = 0.0;
@@ -964,7 +979,7 @@ __device__ __forceinline__ bool weight_phase(Ctx &c, double *s_w, long long *s_q
             const uint32_t j = threadIdx.x * DP + k;
             d[k] = j < nd ? __ldcg(dots + j) : 0.0;
         }
-        seg_fold<DP, kThreads>(c, s_q, nd,
+        seg_fold<THR, DP, THR>(c, s_q, nd,
             [&d](int k) {
                 double x = d[0];
 #pragma unroll
@@ -1062,12 +1077,12 @@ __device__ __forceinline__ void count_reps(const U &u, uint64_t N, uint32_t R, u
 // weight i.  ubuf: global memory for the uniforms of the sorted and stratified
 // sequences.  known (nullable): fold_approx of the weights.  The counts go to
 // s_q (each in its thread's place), the number of uniforms used to *used.
-template <int PER, class Canon, class Again>
+template <int THR, int PER, class Canon, class Again>
 __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s_q, uint64_t N, uint64_t M,
     int scheme, const Canon &canon, const Again &again, double *ubuf, const Approx *known, uint64_t *used,
     unsigned long long *ties)
 {
-    const uint64_t i0 = (static_cast<uint64_t>(c.tile) * kThreads + threadIdx.x) * PER;
+    const uint64_t i0 = (static_cast<uint64_t>(c.tile) * THR + threadIdx.x) * PER;
     const int seq = scheme % 3;
     uint64_t R = M;
     double before = 0.0, total, mul = 1.0;
@@ -1082,14 +1097,14 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
             if (i0 + k < N) acc += static_cast<long long>(static_cast<uint64_t>(ip));
         }
         long long e0, e1, t0, t1;
-        scan_two(c, acc, 0, e0, e1, t0, t1);
+        scan_two<THR>(c, acc, 0, e0, e1, t0, t1);
         if (c.T > 1) {
             unsigned long long x[1] = {static_cast<unsigned long long>(t0)};
             if (!exchange(c, x, false)) return false;
-            scan_two(c, static_cast<long long>(x[0]), 0, e0, e1, t0, t1);
+            scan_two<THR>(c, static_cast<long long>(x[0]), 0, e0, e1, t0, t1);
         }
         R = static_cast<uint64_t>(t0) <= M ? M - static_cast<uint64_t>(t0) : 0;
-        if (!fold_approx<PER>(c, s_v, ap) || !fold_grid<PER, false>(c, s_v, s_q, N, ap, &total, &before)) return false;
+        if (!fold_approx<THR, PER>(c, s_v, ap) || !fold_grid<THR, PER, false>(c, s_v, s_q, N, ap, &total, &before)) return false;
         mul = __ddiv_rn(1.0, total);
     }
     *used = R;
@@ -1099,7 +1114,7 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
             const uint64_t j = i0 + k;
             s_v[at<PER>(k)] = j < R ? -__ddiv_rn(dd::log(canon(j)), static_cast<double>(R - j)) : 0.0;
         }
-        if (!fold_approx<PER>(c, s_v, ap) || !fold_grid<PER, true>(c, s_v, s_q, R, ap, &total, &before)) return false;
+        if (!fold_approx<THR, PER>(c, s_v, ap) || !fold_grid<THR, PER, true>(c, s_v, s_q, R, ap, &total, &before)) return false;
 #pragma unroll 1
         for (int k = 0; k < PER; ++k)
             if (i0 + k < R) ubuf[i0 + k] = __dsub_rn(1.0, exp_rn(-s_v[at<PER>(k)]));
@@ -1129,10 +1144,10 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
         }
         if (known && scheme < 3) {
             ap = *known;
-        } else if (!fold_approx<PER>(c, s_v, ap)) {
+        } else if (!fold_approx<THR, PER>(c, s_v, ap)) {
             return false;
         }
-        if (!fold_grid<PER, true>(c, s_v, s_q, N - 1, ap, &total, &before)) return false;
+        if (!fold_grid<THR, PER, true>(c, s_v, s_q, N - 1, ap, &total, &before)) return false;
         if (seq == 2) {
             const double delta = __ddiv_rn(1.0, static_cast<double>(R));
             const double ud = __dmul_rn(canon(0), delta);
@@ -1170,12 +1185,12 @@ __device__ __forceinline__ bool resample_phase(Ctx &c, double *s_v, long long *s
 // as a rule they lie in the tile itself or its neighbours, whose prefixes are
 // staged in shared memory and searched there (a search of the prefixes in L2
 // from every empty slot measured 14 us at 2^20 particles against 4).
-template <int PER, class Keep, class Copy>
+template <int THR, int PER, class Keep, class Copy>
 __device__ __forceinline__ bool index_phase(Ctx &c, double *s_v, long long *s_q, uint64_t N, uint64_t M,
     uint32_t *surp, const Keep &keep, const Copy &copy)
 {
     Shared *sh = c.sh;
-    constexpr uint32_t TILE = kThreads * PER;
+    constexpr uint32_t TILE = THR * PER;
     constexpr uint32_t kStageTiles = 4 * padded(TILE) / TILE;  // tiles of prefixes that fit the two arrays
     const uint64_t base = static_cast<uint64_t>(c.tile) * TILE, i0 = base + threadIdx.x * PER, K = min(N, M);
     const auto surplus = [K](uint64_t i, long long rep) { return i < K ? (rep != 0 ? rep - 1 : 0) : rep; };
@@ -1192,7 +1207,7 @@ __device__ __forceinline__ bool index_phase(Ctx &c, double *s_v, long long *s_q,
         if (i < N) s += surplus(i, rep);
     }
     long long E, S, te, ts;
-    scan_two(c, e, s, E, S, te, ts);
+    scan_two<THR>(c, e, s, E, S, te, ts);
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
         const uint64_t i = i0 + k;
@@ -1210,7 +1225,7 @@ __device__ __forceinline__ bool index_phase(Ctx &c, double *s_v, long long *s_q,
             ps += static_cast<long long>(xs[1][t]);
         }
     } else if (c.T > 1) {
-        scan_two(c, static_cast<long long>(x[0]), static_cast<long long>(x[1]), pe, ps, t0, t1);
+        scan_two<THR>(c, static_cast<long long>(x[0]), static_cast<long long>(x[1]), pe, ps, t0, t1);
     }
     if (threadIdx.x < c.T) {
         sh->pw[threadIdx.x] = static_cast<uint32_t>(pe);
@@ -1218,7 +1233,7 @@ __device__ __forceinline__ bool index_phase(Ctx &c, double *s_v, long long *s_q,
     }
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
-        const uint32_t o = k * kThreads + threadIdx.x;
+        const uint32_t o = k * THR + threadIdx.x;
         if (base + o < K && s_q[pad(o)] != 0) keep(base + o);
     }
     __syncthreads();
@@ -1243,10 +1258,10 @@ __device__ __forceinline__ bool index_phase(Ctx &c, double *s_v, long long *s_q,
     if (staged && ne) {
         const uint4 *src = reinterpret_cast<const uint4 *>(surp + static_cast<size_t>(ta) * TILE);
         uint4 *dst = reinterpret_cast<uint4 *>(st);
-        for (uint32_t k = threadIdx.x; k < (tb - ta + 1) * (TILE / 4); k += kThreads) dst[k] = __ldcg(src + k);
+        for (uint32_t k = threadIdx.x; k < (tb - ta + 1) * (TILE / 4); k += THR) dst[k] = __ldcg(src + k);
     }
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < ne; k += kThreads) {
+    for (uint32_t k = threadIdx.x; k < ne; k += THR) {
         const uint32_t q = E0 + k;
         // the source: the last particle of its tile with surp <= q - (before the tile)
         uint32_t t = ta;

@@ -1,7 +1,7 @@
 """The cooperative SMC kernels (csrc/smc_coop.cuh) at the sizes where their
 tiling changes: one tile (1024), a cluster of tiles (8 x 1024), one tile per SM
-(148 x 1024), 4096-element tiles one and two per SM, and just past what the chip
-holds (296 x 4096, the multi-kernel path); with the weights that send the exact
+(148 x 1024), the tiles of 4096, 7168 and 8192 elements, and just past what the chip
+holds (148 x 8192, the multi-kernel path); with the weights that send the exact
 fold through its event loop, and genealogies whose copies come from far tiles.
 Bars as in test_gpu_smc.py and test_gpu_pf.py: weights within 2 ULP, ESS within
 1e-13, counts, parents and engine states identical.
@@ -15,8 +15,8 @@ pytestmark = pytest.mark.gpu
 
 import oracle as O  # noqa: E402
 
-EDGES = [1, 2, 1023, 1024, 1025, 2049, 8192, 8193, 148 * 1024, 148 * 1024 + 1, 148 * 4096 + 5, 296 * 4096,
-         296 * 4096 + 1]
+EDGES = [1, 2, 1023, 1024, 1025, 2049, 8192, 8193, 148 * 1024, 148 * 1024 + 1, 148 * 4096 + 5, 148 * 7168, 148 * 8192,
+         148 * 8192 + 1]
 
 
 @pytest.fixture(scope="module")
