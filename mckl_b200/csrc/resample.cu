@@ -469,16 +469,31 @@ __global__ void __launch_bounds__(kFillThreads) k_rep_fill(uint64_t N, uint64_t 
 }
 
 // idx[i] == i for every occupied slot, and a copy reads only occupied slots,
-// so no slot is read after it is written
+// so no slot is read after it is written.  The chain idx -> source -> slot is
+// all latency: two slots per thread and up to four dimensions of each are read
+// before anything is stored (2^20 x 4 doubles: 31.7 -> SEL_NOW us).
 template <typename T>
 __global__ void k_select_inplace(uint64_t N, uint64_t dim, const uint64_t *idx, T *state)
 {
     pdl_wait();
-    GRID_LOOP(i, N)
-    {
-        const uint64_t src = idx[i];
-        if (src != i)
-            for (uint64_t d = 0; d < dim; ++d) state[d * N + i] = state[d * N + src];
+    constexpr int kDims = 4;
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    for (uint64_t i0 = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i0 < N; i0 += 2 * stride) {
+        const uint64_t i1 = i0 + stride;
+        const uint64_t s0 = idx[i0], s1 = i1 < N ? idx[i1] : i1;
+        for (uint64_t d = 0; d < dim; d += kDims) {
+            T a[kDims], b[kDims];
+#pragma unroll
+            for (int k = 0; k < kDims; ++k) {
+                if (d + k < dim && s0 != i0) a[k] = state[(d + k) * N + s0];
+                if (d + k < dim && s1 != i1) b[k] = state[(d + k) * N + s1];
+            }
+#pragma unroll
+            for (int k = 0; k < kDims; ++k) {
+                if (d + k < dim && s0 != i0) state[(d + k) * N + i0] = a[k];
+                if (d + k < dim && s1 != i1) state[(d + k) * N + i1] = b[k];
+            }
+        }
     }
 }
 

@@ -250,10 +250,26 @@ __device__ __forceinline__ bool store_warp32(R *out, uint64_t b, uint64_t nblk, 
     return true;
 }
 
-// Aligned shape: nblk whole blocks starting at counter `base`; block b feeds
-// outputs [b * OPB, (b + 1) * OPB).  `out` is 16-byte aligned.
-template <class G, typename W, class F, int THREADS = 256>
-__global__ void __launch_bounds__(THREADS) k_blocks(G g, Ctr base, uint64_t nblk, typename F::out_t *out, F f)
+// The outputs of block b of a launch: a vector, or the first `rem` of the block
+// after the last whole one.
+template <typename R, int N>
+__device__ __forceinline__ void store_block(R *out, uint64_t b, uint64_t nblk, uint32_t rem, const R (&v)[N])
+{
+    if (b < nblk) {
+        store_aligned<R, N>(out + b * N, v);
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            if (q < static_cast<int>(rem)) out[b * N + q] = v[q];
+    }
+}
+
+// Aligned shape: nblk whole blocks starting at counter `base`, and the first
+// `rem` outputs of one more; block b feeds outputs [b * OPB, (b + 1) * OPB).
+// `out` is 16-byte aligned.
+template <class G, typename W, class F, int THREADS = 256, bool REM = true>
+__global__ void __launch_bounds__(THREADS) k_blocks(G g, Ctr base, uint64_t nblk, uint32_t rem,
+    typename F::out_t *out, F f)
 {
     using R = typename F::out_t;
     constexpr int WPB = G::kWords / WordView<W>::kPer32;  // words per block
@@ -264,12 +280,12 @@ __global__ void __launch_bounds__(THREADS) k_blocks(G g, Ctr base, uint64_t nblk
     // overlap with the stores in flight; one for the transforms whose
     // per-value math (double-double log) needs the registers
     constexpr int U = F::kCheap ? 4 : 1;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b0 < nblk; b0 += U * stride) {
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x, total = REM ? nblk + (rem ? 1 : 0) : nblk;
+    for (uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b0 < total; b0 += U * stride) {
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             const uint64_t b = b0 + i * stride;
-            if (b >= nblk) break;
+            if (b >= total) break;
             uint32_t blk[G::kWords];
             g.block(ctr_add(base, b, G::kCtrWords), blk);
             W w[WPB];
@@ -283,26 +299,31 @@ __global__ void __launch_bounds__(THREADS) k_blocks(G g, Ctr base, uint64_t nblk
             if constexpr (sizeof(R) * OPB == 32 && F::kCheap && std::is_same<G, PhiloxGen>::value) {
                 if (store_warp32<R, OPB>(out, b, nblk, o)) continue;
             }
-            store_aligned<R, OPB>(out + b * OPB, o);
+            if constexpr (REM) {
+                store_block<R, OPB>(out, b, nblk, rem, o);
+            } else {
+                store_aligned<R, OPB>(out + b * OPB, o);
+            }
         }
     }
 }
 
 // k_blocks for Philox launches whose block counters differ only in their low
 // word (PhiloxLo: the counter-independent products folded once per launch).
-template <typename W, class F>
-__global__ void __launch_bounds__(256) k_blocks_plo(PhiloxLo p, uint64_t nblk, typename F::out_t *out, F f)
+template <typename W, class F, bool REM>
+__global__ void __launch_bounds__(256) k_blocks_plo(PhiloxLo p, uint64_t nblk, uint32_t rem,
+    typename F::out_t *out, F f)
 {
     using R = typename F::out_t;
     constexpr int WPB = PhiloxGen::kWords / WordView<W>::kPer32;
     constexpr int OPB = WPB / F::kIn;
     constexpr int U = F::kCheap ? 4 : 1;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b0 < nblk; b0 += U * stride) {
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x, total = REM ? nblk + (rem ? 1 : 0) : nblk;
+    for (uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b0 < total; b0 += U * stride) {
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             const uint64_t b = b0 + i * stride;
-            if (b >= nblk) break;
+            if (b >= total) break;
             uint32_t blk[PhiloxGen::kWords];
             p.block(static_cast<uint32_t>(b), blk);
             W w[WPB];
@@ -314,8 +335,63 @@ __global__ void __launch_bounds__(256) k_blocks_plo(PhiloxLo p, uint64_t nblk, t
             if constexpr (sizeof(R) * OPB == 32 && F::kCheap) {
                 if (store_warp32<R, OPB>(out, b, nblk, o)) continue;
             }
-            store_aligned<R, OPB>(out + b * OPB, o);
+            if constexpr (REM) {
+                store_block<R, OPB>(out, b, nblk, rem, o);
+            } else {
+                store_aligned<R, OPB>(out + b * OPB, o);
+            }
         }
+    }
+}
+
+// Shifted shape: outputs [0, ngroups OPB + rem) from a stream that starts at word
+// `off` (not 0) of block `base`, one word per output, `out` 16-byte aligned.
+// Every lane transforms a block of its own; the output group of OPB values at
+// block b holds the block's values from `off` on and the first `off` of the next
+// block, which the next lane has: the lanes shift their values down by powers
+// of two with shuffles and store whole vectors.  A warp's last lane only serves
+// the one before it (31 groups for 32 blocks).  Against the staged shape: no
+// shared memory, no barriers, vector stores (5e6 single-precision Exponentials
+// from ARS at an offset of one word: 31.0 -> 24.6 us, with the wider table
+// set-up).
+template <class G, typename W, class F, int THREADS = 256>
+__global__ void __launch_bounds__(THREADS) k_shifted(G g, Ctr base, uint32_t off, uint64_t ngroups,
+    uint32_t rem, typename F::out_t *out, F f)
+{
+    using R = typename F::out_t;
+    constexpr int WPB = G::kWords / WordView<W>::kPer32;
+    g.prepare();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (THREADS / 32), total = ngroups + (rem ? 1 : 0);
+    for (uint64_t w = static_cast<uint64_t>(blockIdx.x) * (THREADS / 32) + threadIdx.x / 32; w * 31 < total;
+         w += warps) {
+        const uint64_t b = w * 31 + lane;  // block `total` serves the last group
+        R o[WPB];
+        if (b <= total) {
+            uint32_t blk[G::kWords];
+            g.block(ctr_add(base, b, G::kCtrWords), blk);
+            W v[WPB];
+#pragma unroll
+            for (int j = 0; j < WPB; ++j) v[j] = WordView<W>::get(blk, j);
+#pragma unroll
+            for (int j = 0; j < WPB; ++j) o[j] = f(v + j);
+        } else {
+#pragma unroll
+            for (int j = 0; j < WPB; ++j) o[j] = R(0);
+        }
+#pragma unroll
+        for (int s = 1; s < WPB; s <<= 1) {
+            if (off & s) {  // the same for every lane
+                R t[WPB];
+#pragma unroll
+                for (int j = 0; j < s; ++j) t[j] = __shfl_down_sync(0xffffffffu, o[j], 1);
+#pragma unroll
+                for (int j = 0; j + s < WPB; ++j) o[j] = o[j + s];
+#pragma unroll
+                for (int j = 0; j < s; ++j) o[WPB - s + j] = t[j];
+            }
+        }
+        if (lane < 31 && b < total) store_block<R, WPB>(out, b, ngroups, rem, o);
     }
 }
 
@@ -462,39 +538,50 @@ static int launch_words(const G &g, const Ctr &B, uint32_t off, uint64_t n, type
     // ARS: 32 KiB of table per CTA bounds residency at 6 CTAs per SM
     const int ctas = std::is_same<G, ArsGen>::value ? 6 : 8;
     if (aligned) {
-        const uint64_t nblk = n / OPB;
-        bool done_blocks = false;
+        const uint64_t nblk = n / OPB, total = (n + OPB - 1) / OPB;
+        const uint32_t rem = static_cast<uint32_t>(n % OPB);
         if constexpr (std::is_same<G, PhiloxGen>::value) {
             // no carry out of the low counter word within this launch
-            if (nblk && (B.w[0] & 0xffffffffull) + (nblk - 1) <= 0xffffffffull) {
-                k_blocks_plo<W, F><<<grid_for(nblk, 256, ctas), 256, 0, s>>>(PhiloxLo::make(g, B), nblk, out, f);
+            if ((B.w[0] & 0xffffffffull) + (total - 1) <= 0xffffffffull) {
+                // (the store of a partial block costs the whole fill 4 %)
+                const PhiloxLo p = PhiloxLo::make(g, B);
+                const unsigned grid = grid_for(total, 256, ctas);
+                if (rem) {
+                    k_blocks_plo<W, F, true><<<grid, 256, 0, s>>>(p, nblk, rem, out, f);
+                } else {
+                    k_blocks_plo<W, F, false><<<grid, 256, 0, s>>>(p, nblk, 0, out, f);
+                }
                 MB_LAUNCH_CHECK();
-                done_blocks = true;
+                return MCKL_B200_OK;
             }
         }
         if constexpr (std::is_same<G, ArsGen>::value) {
             // ARS with four round tables: one 1024-thread CTA per SM
-            if (nblk) {
-                MB_CUDA(allow_dyn_smem(k_blocks<ArsGen4, W, F, 1024>, ArsGen4::kDynSmem));
-                k_blocks<ArsGen4, W, F, 1024><<<grid_for(nblk, 1024, 1), 1024, ArsGen4::kDynSmem, s>>>(
-                    ArsGen4::from(g), B, nblk, out, f);
-                MB_LAUNCH_CHECK();
-                done_blocks = true;
-            }
-        }
-        if (nblk && !done_blocks) {
+            MB_CUDA(allow_dyn_smem(k_blocks<ArsGen4, W, F, 1024>, ArsGen4::kDynSmem));
+            k_blocks<ArsGen4, W, F, 1024><<<grid_for(total, 1024, 1), 1024, ArsGen4::kDynSmem, s>>>(
+                ArsGen4::from(g), B, nblk, rem, out, f);
+        } else {
             MB_CUDA(allow_dyn_smem(k_blocks<G, W, F>, G::kDynSmem));
-            k_blocks<G, W, F><<<grid_for(nblk, 256, ctas), 256, G::kDynSmem, s>>>(g, B, nblk, out, f);
-            MB_LAUNCH_CHECK();
+            k_blocks<G, W, F><<<grid_for(total, 256, ctas), 256, G::kDynSmem, s>>>(g, B, nblk, rem, out, f);
         }
-        const uint64_t done = nblk * OPB;
-        if (done < n) {
-            const Ctr B2 = ctr_add(B, nblk, G::kCtrWords);
-            MB_CUDA(allow_dyn_smem(k_staged<G, W, F, 256>, G::kDynSmem));
-            k_staged<G, W, F, 256><<<1, 256, G::kDynSmem, s>>>(g, B2, 0, n - done, out + done, f);
-            MB_LAUNCH_CHECK();
-        }
+        MB_LAUNCH_CHECK();
         return MCKL_B200_OK;
+    }
+    if constexpr (F::kIn == 1) {
+        // enough groups for the shifted shape to pay for its last partial warp
+        if (reinterpret_cast<uintptr_t>(out) % 16 == 0 && n >= 4096) {
+            const uint64_t ng = n / WPB, warps = (ng + 1 + 30) / 31;
+            const uint32_t rem = static_cast<uint32_t>(n % WPB);
+            if constexpr (std::is_same<G, ArsGen>::value) {
+                MB_CUDA(allow_dyn_smem(k_shifted<ArsGen4, W, F, 1024>, ArsGen4::kDynSmem));
+                k_shifted<ArsGen4, W, F, 1024><<<grid_for(warps * 32, 1024, 1), 1024, ArsGen4::kDynSmem, s>>>(
+                    ArsGen4::from(g), B, off, ng, rem, out, f);
+            } else {
+                k_shifted<G, W, F><<<grid_for(warps * 32, 256, ctas), 256, 0, s>>>(g, B, off, ng, rem, out, f);
+            }
+            MB_LAUNCH_CHECK();
+            return MCKL_B200_OK;
+        }
     }
     const uint64_t tiles = (static_cast<uint64_t>(off) + n * F::kIn + 256 * WPB - 1) / (256 * WPB);
     MB_CUDA(allow_dyn_smem(k_staged<G, W, F, 256>, G::kDynSmem));
