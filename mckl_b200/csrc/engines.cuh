@@ -77,13 +77,11 @@ struct PhiloxGen {
     }
 };
 
-__host__ __device__ inline uint32_t mulhi32(uint32_t a, uint32_t b)
+__host__ __device__ __forceinline__ void mul_wide(uint32_t a, uint32_t b, uint32_t &hi, uint32_t &lo)
 {
-#ifdef __CUDA_ARCH__
-    return __umulhi(a, b);
-#else
-    return static_cast<uint32_t>((static_cast<uint64_t>(a) * b) >> 32);
-#endif
+    const uint64_t p = static_cast<uint64_t>(a) * b;
+    hi = static_cast<uint32_t>(p >> 32);
+    lo = static_cast<uint32_t>(p);
 }
 
 // Philox blocks of one launch whose counters differ only in the low 32-bit
@@ -91,7 +89,11 @@ __host__ __device__ inline uint32_t mulhi32(uint32_t a, uint32_t b)
 // depend on the block, so neither do the first round's outputs s0' and s1',
 // nor the second round's product of s0'.  Those are folded once per launch
 // (make); a block then takes 36 of the 40 multiply halves.  The output is
-// the same as PhiloxGen::block on the full counter.
+// the same as PhiloxGen::block on the full counter.  The multiply pipe is the
+// limit; a round's products are taken whole, one 64-bit multiply each, which
+// issues in two thirds of the time of its halves (2^26 words 48.5 -> 43.2 us back
+// to back, one block per thread and iteration; with four the kernel is slower, and
+// so are the filters' kernels with whole products, for want of registers).
 struct PhiloxLo {
     uint32_t lo;            // s0 of block 0 of the launch
     uint32_t k1s3;          // k1 ^ s3 (first round, third word)
@@ -103,14 +105,16 @@ struct PhiloxLo {
         const uint32_t s1 = static_cast<uint32_t>(base.w[0] >> 32);
         const uint32_t s2 = static_cast<uint32_t>(base.w[1]);
         const uint32_t s3 = static_cast<uint32_t>(base.w[1] >> 32);
-        const uint32_t s0p = g.k0 ^ s1 ^ mulhi32(s2, 0xCD9E8D57u);
-        const uint32_t s1p = s2 * 0xCD9E8D57u;
+        uint32_t h1, s1p, h2, l2;
+        mul_wide(s2, 0xCD9E8D57u, h1, s1p);
+        const uint32_t s0p = g.k0 ^ s1 ^ h1;
+        mul_wide(s0p, 0xD2511F53u, h2, l2);
         PhiloxLo p;
         p.lo = static_cast<uint32_t>(base.w[0]);
         p.k1s3 = g.k1 ^ s3;
         p.ca = (g.k0 + 0x9E3779B9u) ^ s1p;
-        p.cb = (g.k1 + 0xBB67AE85u) ^ mulhi32(s0p, 0xD2511F53u);
-        p.lo0c = s0p * 0xD2511F53u;
+        p.cb = (g.k1 + 0xBB67AE85u) ^ h2;
+        p.lo0c = l2;
         p.a2 = g.k0 + 2u * 0x9E3779B9u;
         p.b2 = g.k1 + 2u * 0xBB67AE85u;
         return p;
@@ -120,19 +124,19 @@ struct PhiloxLo {
     __host__ __device__ __forceinline__ void block(uint32_t i, uint32_t out[4]) const
     {
         const uint32_t s0 = lo + i;
-        const uint32_t t2 = k1s3 ^ mulhi32(s0, 0xD2511F53u);  // first round
-        const uint32_t t3 = s0 * 0xD2511F53u;
-        uint32_t x0 = ca ^ mulhi32(t2, 0xCD9E8D57u);  // second round
-        uint32_t x1 = t2 * 0xCD9E8D57u;
+        uint32_t h, t3, x1;
+        mul_wide(s0, 0xD2511F53u, h, t3);  // first round
+        const uint32_t t2 = k1s3 ^ h;
+        mul_wide(t2, 0xCD9E8D57u, h, x1);  // second round
+        uint32_t x0 = ca ^ h;
         uint32_t x2 = cb ^ t3;
         uint32_t x3 = lo0c;
         uint32_t a = a2, b = b2;
 #pragma unroll
         for (int r = 2; r < 10; ++r) {
-            const uint32_t hi2 = mulhi32(x2, 0xCD9E8D57u);
-            const uint32_t lo2 = x2 * 0xCD9E8D57u;
-            const uint32_t hi0 = mulhi32(x0, 0xD2511F53u);
-            const uint32_t lo0 = x0 * 0xD2511F53u;
+            uint32_t hi2, lo2, hi0, lo0;
+            mul_wide(x2, 0xCD9E8D57u, hi2, lo2);
+            mul_wide(x0, 0xD2511F53u, hi0, lo0);
             x0 = a ^ x1 ^ hi2;
             x1 = lo2;
             x2 = b ^ x3 ^ hi0;

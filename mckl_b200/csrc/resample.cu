@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(kFillThreads) k_rep_fill(uint64_t N, uint64_t 
 // idx[i] == i for every occupied slot, and a copy reads only occupied slots,
 // so no slot is read after it is written.  The chain idx -> source -> slot is
 // all latency: two slots per thread and up to four dimensions of each are read
-// before anything is stored (2^20 x 4 doubles: 31.7 -> SEL_NOW us).
+// before anything is stored.
 template <typename T>
 __global__ void k_select_inplace(uint64_t N, uint64_t dim, const uint64_t *idx, T *state)
 {

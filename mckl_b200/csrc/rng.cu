@@ -311,35 +311,33 @@ __global__ void __launch_bounds__(THREADS) k_blocks(G g, Ctr base, uint64_t nblk
 // k_blocks for Philox launches whose block counters differ only in their low
 // word (PhiloxLo: the counter-independent products folded once per launch).
 template <typename W, class F, bool REM>
-__global__ void __launch_bounds__(256) k_blocks_plo(PhiloxLo p, uint64_t nblk, uint32_t rem,
+__global__ void __launch_bounds__(256) k_blocks_plo(PhiloxLo p, uint32_t nblk, uint32_t rem,
     typename F::out_t *out, F f)
 {
     using R = typename F::out_t;
     constexpr int WPB = PhiloxGen::kWords / WordView<W>::kPer32;
     constexpr int OPB = WPB / F::kIn;
-    constexpr int U = F::kCheap ? 4 : 1;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x, total = REM ? nblk + (rem ? 1 : 0) : nblk;
-    for (uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; b0 < total; b0 += U * stride) {
+    const uint32_t stride = gridDim.x * blockDim.x, total = REM ? nblk + (rem ? 1 : 0) : nblk;
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+    // 32-bit block numbers (total < 2^32): the loop's arithmetic is on the same
+    // pipes as the generator's
+    for (uint32_t b = first, left = first < total ? total - first : 0; left > 0;
+         left = left > stride ? left - stride : 0, b += stride) {
+        uint32_t blk[PhiloxGen::kWords];
+        p.block(b, blk);
+        W w[WPB];
 #pragma unroll
-        for (int i = 0; i < U; ++i) {
-            const uint64_t b = b0 + i * stride;
-            if (b >= total) break;
-            uint32_t blk[PhiloxGen::kWords];
-            p.block(static_cast<uint32_t>(b), blk);
-            W w[WPB];
+        for (int j = 0; j < WPB; ++j) w[j] = WordView<W>::get(blk, j);
+        R o[OPB];
 #pragma unroll
-            for (int j = 0; j < WPB; ++j) w[j] = WordView<W>::get(blk, j);
-            R o[OPB];
-#pragma unroll
-            for (int j = 0; j < OPB; ++j) o[j] = f(w + j * F::kIn);
-            if constexpr (sizeof(R) * OPB == 32 && F::kCheap) {
-                if (store_warp32<R, OPB>(out, b, nblk, o)) continue;
-            }
-            if constexpr (REM) {
-                store_block<R, OPB>(out, b, nblk, rem, o);
-            } else {
-                store_aligned<R, OPB>(out + b * OPB, o);
-            }
+        for (int j = 0; j < OPB; ++j) o[j] = f(w + j * F::kIn);
+        if constexpr (sizeof(R) * OPB == 32 && F::kCheap) {
+            if (store_warp32<R, OPB>(out, b, nblk, o)) continue;
+        }
+        if constexpr (REM) {
+            store_block<R, OPB>(out, b, nblk, rem, o);
+        } else {
+            store_aligned<R, OPB>(out + static_cast<uint64_t>(b) * OPB, o);
         }
     }
 }
@@ -542,14 +540,14 @@ static int launch_words(const G &g, const Ctr &B, uint32_t off, uint64_t n, type
         const uint32_t rem = static_cast<uint32_t>(n % OPB);
         if constexpr (std::is_same<G, PhiloxGen>::value) {
             // no carry out of the low counter word within this launch
-            if ((B.w[0] & 0xffffffffull) + (total - 1) <= 0xffffffffull) {
+            if ((B.w[0] & 0xffffffffull) + total <= 0xffffffffull) {
                 // (the store of a partial block costs the whole fill 4 %)
                 const PhiloxLo p = PhiloxLo::make(g, B);
                 const unsigned grid = grid_for(total, 256, ctas);
                 if (rem) {
-                    k_blocks_plo<W, F, true><<<grid, 256, 0, s>>>(p, nblk, rem, out, f);
+                    k_blocks_plo<W, F, true><<<grid, 256, 0, s>>>(p, static_cast<uint32_t>(nblk), rem, out, f);
                 } else {
-                    k_blocks_plo<W, F, false><<<grid, 256, 0, s>>>(p, nblk, 0, out, f);
+                    k_blocks_plo<W, F, false><<<grid, 256, 0, s>>>(p, static_cast<uint32_t>(nblk), 0, out, f);
                 }
                 MB_LAUNCH_CHECK();
                 return MCKL_B200_OK;
