@@ -632,8 +632,7 @@ class CounterEngine:
 
     def copy(self):
         other = type(self).__new__(type(self))
-        other.state = EngineState()
-        ctypes.pointer(other.state)[0] = self.state
+        other.state = EngineState.from_buffer_copy(self.state)
         return other
 
     def state_tuple(self):
@@ -702,25 +701,39 @@ ENGINES = {"Philox4x32": Philox4x32, "Philox4x32_64": Philox4x32_64, "Threefry4x
 # ---------------------------------------------------------------------------
 # tensors and streams
 # ---------------------------------------------------------------------------
-def _torch():
-    import torch  # local: the library itself does not need torch
+# A small draw costs the host more than the GPU, so what every call does here is
+# kept short: the module and torch's raw stream lookup are looked up once, and
+# addresses are passed as integers.
+_torch_module = None
+_raw_stream = None
 
-    return torch
+
+def _torch():
+    global _torch_module, _raw_stream
+    if _torch_module is None:
+        import torch  # local: the library itself does not need torch
+
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream_ptr(stream=None) -> int:
-    torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+    if stream is not None:
+        return int(stream.cuda_stream)
+    torch = _torch_module or _torch()
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return int(torch.cuda.current_stream().cuda_stream)
 
 
-def _check_out(r, n: int, itemsize: int):
-    torch = _torch()
+def _check_out(r, n: int, itemsize: int) -> int:
+    torch = _torch_module or _torch()
     if not isinstance(r, torch.Tensor) or not (r.is_cuda or r.is_pinned()):
         raise MCKLB200Error("output must be a CUDA tensor or a pinned host tensor")
     if not r.is_contiguous() or r.element_size() != itemsize or r.numel() < n:
         raise MCKLB200Error("output tensor has the wrong size, dtype width or layout")
-    return ctypes.c_void_p(r.data_ptr())
+    return r.data_ptr()
 
 
 def empty_words(rng: CounterEngine, n: int, device="cuda"):
