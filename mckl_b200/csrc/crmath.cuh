@@ -225,7 +225,7 @@ MB_HD bool log_quick(double x, double *y)
     const long long bits = MB_AS_BITS(x);
     // positive normal doubles only
     if (static_cast<unsigned long long>(bits) - 0x0010000000000000ull >= 0x7fe0000000000000ull) return false;
-    const double e = static_cast<double>(static_cast<int>(bits >> 52) - 1023);
+    const double e = MB_SUB(MB_FROM_BITS(0x4330000000000000ll | (bits >> 52)), 0x1p52 + 1023.0);  // exact
     const double m = MB_FROM_BITS((bits & 0x000fffffffffffffll) | 0x3ff0000000000000ll);
     const int i = static_cast<int>((bits >> 45) & 127);
     const double r = MB_FMA(m, MB_LOGTAB(i, 0), -1.0);  // exact
@@ -329,19 +329,33 @@ static const double kExpTabHost[64][2] = {
 #define MB_EXPTAB(j, k) kExpTabHost[(j)][(k)]
 #endif
 
-// Ziv's rounding test: v.hi = RN(v.hi + v.lo), and v approximates a value
-// to within 2^-62 relative.  True when every value that close rounds to v.hi,
-// i.e. when v.hi is the correctly rounded value.  Below a power of two the
-// gap to the next double is half as wide, so the test uses a quarter ulp on
-// that side.  Zero and subnormal v.hi fail.
-MB_HD bool ziv_ok(const DD &v)
+// Ziv's rounding test: v.hi = RN(v.hi + v.lo), a normal number, approximates a
+// value to within 2^-63 relative.  Both ends of the interval of half-width
+// 2^-62 |v.hi| are rounded; where they round to one double, every value between
+// does, and *y is the correctly rounded value.  Six operations and one compare;
+// the spacing of doubles below a power of two needs no case of its own.
+MB_HD bool ziv_round(const DD &v, double *y)
 {
-    const long long b = MB_AS_BITS(v.hi) & 0x7fffffffffffffffll;  // |v.hi|
-    const double u = MB_MUL(MB_FROM_BITS(b & 0x7ff0000000000000ll), 0x1p-52);  // ulp(v.hi)
-    const bool inward = v.hi > 0.0 ? v.lo < 0.0 : v.lo > 0.0;
-    const double half = ((b & 0x000fffffffffffffll) == 0 && inward) ? MB_MUL(u, 0.25) : MB_MUL(u, 0.5);
-    const double d = v.lo < 0.0 ? -v.lo : v.lo;
-    return MB_ADD(d, MB_MUL(MB_FROM_BITS(b), 0x1p-62)) < half;
+    const double e = MB_MUL(v.hi, 0x1p-62);
+    const double y0 = MB_ADD(v.hi, MB_SUB(v.lo, e));
+    *y = y0;
+    return y0 == MB_ADD(v.hi, MB_ADD(v.lo, e));
+}
+
+// The nearest integer k of a, |a| < 2^31, by the addition of 1.5 2^52 (one
+// addition and one subtraction, where a conversion instruction runs at a quarter
+// of their rate); *k its low 32 bits as an int.
+MB_HD double round_int(double a, int *k)
+{
+    const double t = MB_ADD(a, 0x1.8p52);
+    *k = static_cast<int>(MB_AS_BITS(t));
+    return MB_SUB(t, 0x1.8p52);
+}
+
+// |x|'s upper 32 bits: a range check of a double in integer arithmetic
+MB_HD unsigned abs_hi(double x)
+{
+    return static_cast<unsigned>(MB_AS_BITS(x) >> 32) & 0x7fffffffu;
 }
 
 constexpr double kExpInvL = 0x1.71547652b82fep+6;  // 64 / ln2
@@ -360,12 +374,12 @@ constexpr double kExpL2 = 0x1.cf79abc9e3b3ap-46;   // RN(ln2/64 - kExpL1)
 // correctly rounded exp(x) -- the value the accurate phase returns there
 // too, as the exact result is then far from any rounding midpoint.  About
 // one argument in 500 fails the test and goes to the accurate phase; so do
-// arguments whose result is not a normal double (outside [-708, 709]).
+// arguments whose result may not be a normal double (|x| >= 708).
 MB_HD bool exp_quick(double x, double *y)
 {
-    if (!(x >= -708.0 && x <= 709.0)) return false;
-    const double kd = MB_RINT(MB_MUL(x, kExpInvL));
-    const int k = static_cast<int>(kd);
+    if (abs_hi(x) >= 0x40862000u) return false;  // |x| >= 708, or not a number
+    int k;
+    const double kd = round_int(MB_MUL(x, kExpInvL), &k);
     const double rh0 = MB_FMA(-kd, kExpL1, x);  // exact
     const DD r = two_sum(rh0, MB_MUL(-kd, kExpL2));
     const double rh = r.hi;
@@ -381,9 +395,10 @@ MB_HD bool exp_quick(double x, double *y)
     const DD s = two_sum(Th, a.hi);
     const double t = MB_ADD(s.lo, MB_ADD(a.lo, MB_FMA(Th, p, MB_FMA(Tl, MB_ADD(rh, p), Tl))));
     const DD v = fast_two_sum(s.hi, t);
-    if (!ziv_ok(v)) return false;
-    *y = MB_MUL(v.hi, MB_FROM_BITS(static_cast<long long>(m + 1023) << 52));  // exact: a normal result
-    return true;
+    double y0;
+    const bool ok = ziv_round(v, &y0);
+    *y = MB_MUL(y0, MB_FROM_BITS(static_cast<long long>(m + 1023) << 52));  // exact: a normal result
+    return ok;
 }
 
 // Correctly rounded (see header) exponential: the quick phase, else the
@@ -491,8 +506,10 @@ static const double kSinCosTabHost[52][4] = {
 // otherwise the call goes to the accurate phase.
 MB_HD bool sincos_quick(double x, double *sp, double *cp)
 {
-    if (!(x < 1e5 && x > -1e5)) return false;
-    const double kd = MB_RINT(MB_MUL(x, kTwoOverPi));
+    // 2^-500 <= |x| < 1e5: no zero, no subnormal, no NaN on this path
+    if (abs_hi(x) - 0x20b00000u >= 0x40f86a00u - 0x20b00000u) return false;
+    int quadrant;
+    const double kd = round_int(MB_MUL(x, kTwoOverPi), &quadrant);
     const double t = MB_FMA(-kd, kPio2P1, x);  // exact
     const DD p2 = two_prod(-kd, kPio2P2);
     DD r = two_sum(t, p2.hi);
@@ -502,9 +519,9 @@ MB_HD bool sincos_quick(double x, double *sp, double *cp)
     r = fast_two_sum(r.hi, r.lo);
     const bool neg = r.hi < 0.0;
     const double ah = neg ? -r.hi : r.hi, bl = neg ? -r.lo : r.lo;  // |r| = ah + bl
-    const double jd = MB_RINT(MB_MUL(ah, 64.0));
-    if (!(jd <= 51.0)) return false;
-    const int j = static_cast<int>(jd);
+    int j;
+    const double jd = round_int(MB_MUL(ah, 64.0), &j);
+    if (j > 51) return false;
     const double bh = MB_SUB(ah, MB_MUL(jd, 0.015625));  // exact
     const double w = MB_MUL(bh, bh);
     double Pc = 0x1.a01a01a01a01ap-16;           // 1/40320
@@ -537,15 +554,14 @@ MB_HD bool sincos_quick(double x, double *sp, double *cp)
     tc = MB_FMA(Ch, cm1, tc);
     tc = MB_ADD(MB_SUB(ca.lo, q.lo), tc);
     const DD cv = fast_two_sum(ca.hi, tc);
-    if (!ziv_ok(sv) || !ziv_ok(cv)) return false;
-    const double s = neg ? -sv.hi : sv.hi, c = cv.hi;
-    switch (static_cast<int>(static_cast<long long>(kd) & 3)) {
-        case 0: *sp = s; *cp = c; break;
-        case 1: *sp = c; *cp = -s; break;
-        case 2: *sp = -s; *cp = -c; break;
-        default: *sp = -c; *cp = s; break;
-    }
-    return true;
+    double s, c;
+    const bool oks = ziv_round(sv, &s), okc = ziv_round(cv, &c);
+    // quadrant q: (s, c), (c, -s), (-s, -c), (-c, s); s with r's sign
+    const bool swap = (quadrant & 1) != 0;
+    const long long fs = (neg && !swap) != ((quadrant & 2) != 0), fc = (neg && swap) != (((quadrant + 1) & 2) != 0);
+    *sp = MB_FROM_BITS(MB_AS_BITS(swap ? c : s) ^ static_cast<long long>(static_cast<unsigned long long>(fs) << 63));
+    *cp = MB_FROM_BITS(MB_AS_BITS(swap ? s : c) ^ static_cast<long long>(static_cast<unsigned long long>(fc) << 63));
+    return oks && okc;
 }
 
 // sin and cos of a double, correctly rounded (see header): the quick phase,

@@ -447,78 +447,110 @@ __global__ void __launch_bounds__(256) k_staged(G g, Ctr base, uint32_t off, uin
 
 // ---------------------------------------------------------------------------
 // Normal: one CTA per 8192-byte chunk.  Chunk c uses stream words
-// [c K, c K + K) (relative to the call's first word); word i < K/2 is the
-// radius uniform and word K/2 + i the angle uniform of output pair
-// (c K + i, c K + K/2 + i).
+// [c K, c K + len) (relative to the call's first word), len = K or, for the last
+// chunk of a call, what is left; word i < len / 2 is the radius uniform and word
+// len / 2 + i the angle uniform of output pair (c K + i, c K + len / 2 + i).  An
+// odd call's last value is mean + (sd sqrt(-2 log u)) cos(2 pi v), u and v the two
+// words after the last chunk (random/normal_distribution.hpp:93-100).  All of a
+// call is one launch.
+//
+// Double is bound by instruction issue and the FP64 pipe.  A pair fails the
+// quick phases' rounding tests with probability about 0.008, so one warp
+// iteration in five would take the accurate phases for one lane.  Such pairs are
+// put on a list of the warp instead, and the list is worked off 32 at a time, at
+// the latest when the warp has done its chunks.  CTAs of 128 threads (256 where
+// the generator keeps a table per CTA) wait less at the two barriers of a chunk;
+// calls of few chunks run 512 threads on each.
+// 2^24 + 1 values (Threefry): 176.0 us before, 133.3 now (one CTA size
+// of 256 threads and no list: 173.2).
 // ---------------------------------------------------------------------------
-template <class G, typename W, typename R, int K>
-__global__ void __launch_bounds__(256) k_normal(G g, Ctr base, uint32_t off, uint64_t first_chunk,
-    uint64_t nchunks, uint32_t len, R *out, R mean, R sd)
+template <class G, typename W, typename R, int K, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_normal(G g, Ctr base, uint32_t off, uint64_t nchunks, uint32_t last_len,
+    R *out, R mean, R sd)
 {
     using O = RealOps<R>;
+    constexpr bool kDefer = sizeof(R) == 8;
     constexpr int WPB = G::kWords / WordView<W>::kPer32;
-    constexpr int NB = K / WPB + 1;  // blocks staged per chunk (one extra for misalignment)
+    constexpr int NB = K / WPB + 1;  // blocks staged per chunk (one extra for misalignment or an odd call's two words)
     __shared__ __align__(16) uint32_t st32[NB * G::kWords];
+    // per warp: pairs for the accurate phases, their first output's number with
+    // len / 2 in the upper 16 bits, and their words
+    __shared__ uint64_t l_at[kDefer ? THREADS / 32 : 1][kDefer ? 64 : 1];
+    __shared__ W l_u[kDefer ? THREADS / 32 : 1][kDefer ? 64 : 1], l_v[kDefer ? THREADS / 32 : 1][kDefer ? 64 : 1];
     const W *st = reinterpret_cast<const W *>(st32);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t cnt = 0;  // entries of the warp's list, below 32 between iterations
     g.prepare();
-    const uint32_t nu = len / 2;
-    for (uint64_t cc = blockIdx.x; cc < nchunks; cc += gridDim.x) {
-        const uint64_t c = first_chunk + cc;
+    auto put = [&](uint64_t i, uint64_t j, R lg, R sn, R cs) {
+        R s = O::sqrt(O::mul(static_cast<R>(-2), lg));
+        if (sd != static_cast<R>(1)) s = O::mul(sd, s);
+        if (mean != static_cast<R>(0)) {
+            out[i] = O::fma(s, sn, mean);
+            out[j] = O::fma(s, cs, mean);
+        } else {
+            out[i] = O::mul(s, sn);
+            out[j] = O::mul(s, cs);
+        }
+    };
+    auto work_off = [&](uint32_t n) {  // the list's last n <= 32 entries
+        if constexpr (kDefer) {
+            __syncwarp();
+            cnt -= n;
+            if (lane < n) {
+                const uint64_t at = l_at[warp][cnt + lane], i = at & 0xffffffffffffull;
+                R lg, sn, cs;
+                pair_accurate(O::u01(kOC, l_u[warp][cnt + lane]),
+                    O::mul(O::kTwoPi, O::u01(kOC, l_v[warp][cnt + lane])), &lg, &sn, &cs);
+                put(i, i + (at >> 48), lg, sn, cs);
+            }
+            __syncwarp();
+        }
+    };
+    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const uint32_t len = c + 1 == nchunks ? last_len : K, nu = len / 2;
+        const bool odd = (len & 1u) != 0;
         const uint64_t a0 = static_cast<uint64_t>(off) + c * K;  // absolute word of the chunk start
         const uint64_t b0 = a0 / WPB;
         const uint32_t s0 = static_cast<uint32_t>(a0 % WPB);
-        const int nb = static_cast<int>((s0 + len + WPB - 1) / WPB);
-        for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+        const int nb = static_cast<int>((s0 + len + (odd ? 2 : 0) + WPB - 1) / WPB);
+        for (int i = threadIdx.x; i < nb; i += THREADS) {
             uint32_t blk[G::kWords];
             g.block(ctr_add(base, b0 + i, G::kCtrWords), blk);
             stage_block<G>(st32, i, blk);
         }
         __syncthreads();
-        R *o = out + c * K;
-        for (uint32_t p = threadIdx.x; p < nu; p += blockDim.x) {
-            const R u1 = O::u01(kOC, st[s0 + p]);
-            const R u2 = O::u01(kOC, st[s0 + nu + p]);
-            R s = O::sqrt(O::mul(static_cast<R>(-2), O::log(u1)));
-            R sn, cs;
-            O::sincos(O::mul(O::kTwoPi, u2), &sn, &cs);
-            if (sd != static_cast<R>(1)) s = O::mul(sd, s);
-            if (mean != static_cast<R>(0)) {
-                o[p] = O::fma(s, sn, mean);
-                o[nu + p] = O::fma(s, cs, mean);
-            } else {
-                o[p] = O::mul(s, sn);
-                o[nu + p] = O::mul(s, cs);
+        const uint64_t o = c * K;
+        for (uint32_t p0 = warp * 32; p0 < nu; p0 += THREADS) {
+            const uint32_t p = p0 + lane;
+            bool ok = true;
+            if (p < nu) {
+                R lg, sn, cs;
+                ok = pair_quick(O::u01(kOC, st[s0 + p]), O::mul(O::kTwoPi, O::u01(kOC, st[s0 + nu + p])), &lg, &sn,
+                    &cs);
+                if (ok) put(o + p, o + nu + p, lg, sn, cs);
+            }
+            if constexpr (kDefer) {
+                const uint32_t m = __ballot_sync(0xffffffffu, !ok);
+                if (m) {
+                    if (!ok) {
+                        const uint32_t e = cnt + __popc(m & ((1u << lane) - 1u));
+                        l_at[warp][e] = (o + p) | static_cast<uint64_t>(nu) << 48;
+                        l_u[warp][e] = st[s0 + p];
+                        l_v[warp][e] = st[s0 + nu + p];
+                    }
+                    cnt += __popc(m);
+                    if (cnt >= 32) work_off(32);
+                }
             }
         }
-        if ((len & 1u) && threadIdx.x == 0) {
-            o[len - 1] = O::u01(kOC, st[s0 + len - 1]);  // raw U01OC, as the reference leaves it
+        if (odd && threadIdx.x == THREADS - 1) {
+            const R a = O::sqrt(O::mul(static_cast<R>(-2), O::log(O::u01(kOC, st[s0 + len]))));
+            const R cv = O::cos(O::mul(O::kTwoPi, O::u01(kOC, st[s0 + len + 1])));
+            out[o + len - 1] = O::add(mean, O::mul(O::mul(sd, a), cv));
         }
         __syncthreads();
     }
-}
-
-// odd-n fix-up: r[n-1] = mean + (sd * sqrt(-2 log u)) * cos(2 pi v), u and v the
-// two words after the last chunk (random/normal_distribution.hpp:93-100)
-template <class G, typename W, typename R>
-__global__ void k_normal_odd(G g, Ctr base, uint64_t a_u, R *dst, R mean, R sd)
-{
-    using O = RealOps<R>;
-    constexpr int WPB = G::kWords / WordView<W>::kPer32;
-    g.prepare();
-    if (threadIdx.x != 0) return;
-    W wv[2];
-    for (int q = 0; q < 2; ++q) {
-        const uint64_t a = a_u + q;
-        uint32_t blk[G::kWords];
-        g.block(ctr_add(base, a / WPB, G::kCtrWords), blk);
-        wv[q] = WordView<W>::get(blk, static_cast<int>(a % WPB));
-    }
-    const R u = O::u01(kOC, wv[0]);
-    const R v = O::u01(kOC, wv[1]);
-    const R a = O::sqrt(O::mul(static_cast<R>(-2), O::log(u)));
-    const R b = O::mul(sd, a);
-    const R c = O::cos(O::mul(O::kTwoPi, v));
-    *dst = O::add(mean, O::mul(b, c));
+    if (cnt) work_off(cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -667,24 +699,19 @@ static int normal_impl(mckl_b200_engine_t *e, size_t n, R *r, R mean, R sd, void
         using G = decltype(g);
         auto run = [&](auto wtag) {
             using W = decltype(wtag);
-            MB_CUDA(allow_dyn_smem(k_normal<G, W, R, K>, G::kDynSmem));
-            if (m) {
-                k_normal<G, W, R, K><<<grid_for(m * 256, 256, 8), 256, G::kDynSmem, s>>>(g, B, off, 0, m, K, r,
-                    mean, sd);
+            const uint64_t chunks = m + (l ? 1 : 0);
+            if (!chunks) return static_cast<int>(MCKL_B200_OK);
+            auto launch = [&](auto threads) {
+                constexpr int T = decltype(threads)::value;
+                MB_CUDA(allow_dyn_smem(k_normal<G, W, R, K, T>, G::kDynSmem));
+                k_normal<G, W, R, K, T><<<grid_for(chunks * T, T, 2048 / T), T, G::kDynSmem, s>>>(g, B, off, chunks,
+                    static_cast<uint32_t>(l ? l : K), r, mean, sd);
                 MB_LAUNCH_CHECK();
-            }
-            if (l) {
-                k_normal<G, W, R, K><<<1, 256, G::kDynSmem, s>>>(g, B, off, m, 1, static_cast<uint32_t>(l), r,
-                    mean, sd);
-                MB_LAUNCH_CHECK();
-            }
-            if (n % 2) {
-                MB_CUDA(allow_dyn_smem(k_normal_odd<G, W, R>, G::kDynSmem));
-                k_normal_odd<G, W, R><<<1, 32, G::kDynSmem, s>>>(g, B, static_cast<uint64_t>(off) + n, r + n - 1,
-                    mean, sd);
-                MB_LAUNCH_CHECK();
-            }
-            return MCKL_B200_OK;
+                return static_cast<int>(MCKL_B200_OK);
+            };
+            // a chunk or two per SM: its latency counts, one pair per thread
+            if (chunks <= 2 * static_cast<uint64_t>(sm_count())) return launch(std::integral_constant<int, 512>{});
+            return launch(std::integral_constant<int, G::kDynSmem ? 256 : 128>{});
         };
         if (is64(e->kind)) return run(uint64_t{});
         return run(uint32_t{});
