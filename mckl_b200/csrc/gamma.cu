@@ -30,12 +30,20 @@
 
 #include "block_scan.cuh"
 #include "common.cuh"
+#include "crmathf.cuh"
 #include "dispatch.cuh"
 #include "transforms.cuh"
 
 namespace mckl_b200 {
 
 namespace {
+
+// The library functions behind the float operations, out of line: one call in
+// some ten thousand gets here.
+__device__ __noinline__ float lib_log(float a) { return __double2float_rn(::log(static_cast<double>(a))); }
+__device__ __noinline__ float lib_exp(float a) { return __double2float_rn(::exp(static_cast<double>(a))); }
+__device__ __noinline__ float lib_sin(float a) { return __double2float_rn(::sin(static_cast<double>(a))); }
+__device__ __noinline__ float lib_cos(float a) { return __double2float_rn(::cos(static_cast<double>(a))); }
 
 template <typename R>
 struct GOps;
@@ -64,15 +72,25 @@ struct GOps<float> {
     __device__ static float sub(float a, float b) { return __fsub_rn(a, b); }
     __device__ static float div(float a, float b) { return __fdiv_rn(a, b); }
     __device__ static float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-    __device__ static float log(float a) { return __double2float_rn(::log(static_cast<double>(a))); }
-    __device__ static float exp(float a) { return __double2float_rn(::exp(static_cast<double>(a))); }
+    __device__ static float log(float a)
+    {
+        float y;
+        if (!dd::log_float(a, &y)) y = lib_log(a);
+        return y;
+    }
+    __device__ static float exp(float a)
+    {
+        float y;
+        if (!dd::exp_float(a, &y)) y = lib_exp(a);
+        return y;
+    }
     __device__ static float sqrt(float a) { return __fsqrt_rn(a); }
     __device__ static void sincos(float a, float *s, float *c)
     {
-        double sd, cd;
-        ::sincos(static_cast<double>(a), &sd, &cd);
-        *s = __double2float_rn(sd);
-        *c = __double2float_rn(cd);
+        if (!dd::sincos_float(a, s, c)) {
+            *s = lib_sin(a);
+            *c = lib_cos(a);
+        }
     }
 };
 
@@ -248,7 +266,7 @@ __device__ __forceinline__ bool gamma_n_accept(const GammaParam<R> &k, R u, R w,
         *r = O::mul(k.d, v);
         return true;
     }
-    e = O::add(O::div(w2, static_cast<R>(2)), O::mul(k.d, O::add(O::sub(static_cast<R>(1), v), O::log(v))));
+    e = O::add(O::mul(w2, static_cast<R>(0.5)), O::mul(k.d, O::add(O::sub(static_cast<R>(1), v), O::log(v))));
     if (O::log(u) < e) {
         *r = O::mul(k.d, v);
         return true;
@@ -642,7 +660,7 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
             if (u[j] < e) {
                 acc[j] = true;
             } else {
-                const R a = O::div(O::mul(w[j], w[j]), static_cast<R>(2));
+                const R a = O::mul(O::mul(w[j], w[j]), static_cast<R>(0.5));
                 const R b = O::add(O::sub(static_cast<R>(1), vv), O::log(vv));
                 e = O::add(a, O::mul(d, b));
                 acc[j] = O::log(u[j]) < e;
