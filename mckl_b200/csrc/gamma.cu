@@ -55,7 +55,6 @@ struct GOps<double> {
     __device__ static double mul(double a, double b) { return __dmul_rn(a, b); }
     __device__ static double add(double a, double b) { return __dadd_rn(a, b); }
     __device__ static double sub(double a, double b) { return __dsub_rn(a, b); }
-    __device__ static double div(double a, double b) { return __ddiv_rn(a, b); }
     __device__ static double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
     __device__ static double log(double a) { return dd::log(a); }
     __device__ static double exp(double a) { return dd::exp(a); }
@@ -70,7 +69,6 @@ struct GOps<float> {
     __device__ static float mul(float a, float b) { return __fmul_rn(a, b); }
     __device__ static float add(float a, float b) { return __fadd_rn(a, b); }
     __device__ static float sub(float a, float b) { return __fsub_rn(a, b); }
-    __device__ static float div(float a, float b) { return __fdiv_rn(a, b); }
     __device__ static float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     __device__ static float log(float a)
     {
@@ -185,43 +183,23 @@ struct ScalarWords {
     }
 };
 
-// CTA-wide ranks of E predicates per thread in index order, element (t, j)
-// having index t + j THREADS: rank[j] = the number of set elements with a
-// smaller index, *total the CTA count.  Three barriers for all E (one ballot
-// per j; warp 0 scans the E x warps counts).  `sh` holds E THREADS / 32 + 1
-// words (at most 64 + 1).
-template <int THREADS, int E>
-__device__ __forceinline__ void block_rank_multi(const bool (&f)[E], uint32_t *sh, uint32_t (&rank)[E],
-    uint32_t *total)
+// Exclusive ranks of a chunk's flagged values: word q of `mask` has the flags of
+// values 32 q .. 32 q + 31, and pre[q] becomes the number of flags in the words
+// before it, pre[nw] (nw <= 64, at least 1) their total.  Two barriers.
+__device__ __forceinline__ void mask_prefix(const uint32_t *mask, uint32_t *pre, uint32_t nw)
 {
-    constexpr int NW = THREADS / 32, L = E * NW;
-    static_assert(L <= 64, "two counts per lane of warp 0");
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t b[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-        b[j] = __ballot_sync(0xffffffffu, f[j]);
-        if (lane == 0) sh[j * NW + warp] = __popc(b[j]);
-    }
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t a0 = lane < static_cast<uint32_t>(L) ? sh[lane] : 0u;
-        const uint32_t a1 = lane + 32 < static_cast<uint32_t>(L) ? sh[lane + 32] : 0u;
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        const uint32_t a0 = lane < nw ? __popc(mask[lane]) : 0u;
+        const uint32_t a1 = lane + 32 < nw ? __popc(mask[lane + 32]) : 0u;
         const uint32_t s0 = warp_inclusive_sum(a0);
-        const uint32_t t0 = __shfl_sync(0xffffffffu, s0, 31);
-        const uint32_t s1 = warp_inclusive_sum(a1) + t0;
-        const uint32_t t1 = __shfl_sync(0xffffffffu, s1, 31);
-        __syncwarp();
-        if (lane < static_cast<uint32_t>(L)) sh[lane] = s0 - a0;
-        if (lane + 32 < static_cast<uint32_t>(L)) sh[lane + 32] = s1 - a1;
-        if (lane == 0) sh[L] = t1;
+        const uint32_t s1 = warp_inclusive_sum(a1) + __shfl_sync(0xffffffffu, s0, 31);
+        if (lane < nw) pre[lane] = s0 - a0;
+        if (lane + 32 < nw) pre[lane + 32] = s1 - a1;
+        if (lane == 31) pre[nw] = s1;
     }
     __syncthreads();
-    const uint32_t lt = (1u << lane) - 1u;
-#pragma unroll
-    for (int j = 0; j < E; ++j) rank[j] = sh[j * NW + warp] + __popc(b[j] & lt);
-    *total = sh[L];
-    __syncthreads();  // `sh` is rewritten by the next call
 }
 
 // Scalar normal with the cached second variate (random/normal_distribution.hpp:136-153).
@@ -449,30 +427,46 @@ struct GammaTraits {
     static constexpr int K = 8192 / static_cast<int>(sizeof(R));
 };
 
-// Shared memory of the chunk loop (after the generator's own table): the
-// staged words of one chunk, reused for the redraw list of algorithm N.
+// Shared memory of the chunk loop (after the generator's own table): the staged
+// words of one chunk, then one R per value (algorithm N's normals; the candidate
+// values of all but E) and the numbers of the values that algorithm N redraws.
 template <class G, typename W, typename R>
 struct GammaSmem {
     static constexpr int K = GammaTraits<R>::K;
     static constexpr int WPB = G::kWords / WordView<W>::kPer32;
     static constexpr int kStageBlocks = (2 * K + 2) / WPB + 2;
-    static constexpr int kStageBytes = kStageBlocks * G::kWords * 4;
-    static constexpr int kListBytes = K * (4 + 2 * static_cast<int>(sizeof(R)));
-    static constexpr int kMainBytes = ((kStageBytes > kListBytes ? kStageBytes : kListBytes) + 15) / 16 * 16;
-    // plus the batch normals of algorithm N
-    static constexpr int kBytes = kMainBytes + K * static_cast<int>(sizeof(R));
+    static constexpr int kMainBytes = (kStageBlocks * G::kWords * 4 + 15) / 16 * 16;
+    static constexpr int kRedrawAt = kMainBytes + K * static_cast<int>(sizeof(R));
+    static constexpr int kBytes = kRedrawAt + K * 2;
+};
+
+// Flags and ranks of a chunk's values, and per warp the values whose acceptance
+// test needs logarithms.
+template <int THREADS, int K>
+struct GammaFlags {
+    uint32_t acc[K / 32], red[K / 32], pre[K / 32 + 1];
+    uint16_t slow[THREADS / 32][64];
+    uint64_t words;  // words the redraws consumed
 };
 
 // One chunk of n <= K values at stream word `pos`; accepted values go to
 // out[0, m).  Returns m; advances `pos` and `eng` past the chunk's words.
+//
+// Bound by instruction issue and, with few warps, by latency.  The loops over a
+// thread's values are rolled and hand values on through shared memory: unrolled,
+// with the values in registers, their code missed the instruction cache and 80
+// registers left 24 warps on an SM.  The squeeze of algorithm N's test rejects
+// one value in some ten, which is one or more in nearly every warp; those wait on
+// a list of the warp and take their two logarithms 32 at a time.
 template <class G, typename W, typename R, int THREADS, int ALG>
 __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B, uint32_t off, uint64_t &pos,
-    DevEngine<G::kCtrWords> &eng, uint32_t n, R *out, unsigned char *smem, uint32_t *shr, uint64_t *sh_pos)
+    DevEngine<G::kCtrWords> &eng, uint32_t n, R *out, unsigned char *smem, GammaFlags<THREADS, GammaTraits<R>::K> &fl)
 {
     using O = GOps<R>;
     using S = GammaSmem<G, W, R>;
-    constexpr int K = S::K, WPB = S::WPB, EPT = K / THREADS;
-    constexpr uint32_t M = static_cast<uint32_t>(WPB);
+    constexpr int K = S::K, WPB = S::WPB;
+    constexpr uint32_t M = static_cast<uint32_t>(WPB), NW = THREADS / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
     const R d = k.d, c = k.c, beta = k.beta;
     // ---- stage this chunk's words
     const uint64_t nw = (ALG <= 1) ? 2ull * n : (ALG == 2 ? 2ull * n + ((n & 1u) ? 2 : 0) : n);
@@ -488,62 +482,68 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
         for (int q = 0; q < G::kWords; ++q) st32[i * G::kWords + q] = blk[q];
     }
     __syncthreads();
-    R x[EPT];
-    bool acc[EPT];
-    uint32_t got = 0;
     if constexpr (ALG == 3) {
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) {
+        for (uint32_t j = 0; j < (K + THREADS - 1) / THREADS; ++j) {
             const uint32_t i = threadIdx.x + j * THREADS;
             if (i < n) out[i] = O::mul(-beta, O::log(RealOps<R>::u01(kOO, st[s0 + i])));
         }
-        got = n;
-        __syncthreads();
-    } else if constexpr (ALG <= 1) {
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
+        eng.batch(n, K, M);
+        pos += nw;
+        __syncthreads();  // the staged words are rewritten by the next chunk
+        return n;
+    }
+    R *buf = reinterpret_cast<R *>(smem + S::kMainBytes);
+    // value i = 32 q + lane of word q = warp + NW j, j < rounds
+    const uint32_t rounds = (n + THREADS - 1) / THREADS;
+    if constexpr (ALG <= 1) {
+#pragma unroll 1
+        for (uint32_t j = 0; j < rounds; ++j) {
             const uint32_t i = threadIdx.x + j * THREADS;
-            acc[j] = false;
-            if (i >= n) continue;
-            R u = RealOps<R>::u01(kOO, st[s0 + i]);
-            R e = RealOps<R>::u01(kOO, st[s0 + n + i]);
-            if constexpr (ALG == 0) {
-                e = O::mul(static_cast<R>(-1), O::log(e));
-                if (u > d) {
-                    const R t = O::mul(c, O::sub(static_cast<R>(1), u));
-                    u = -O::log(t);
-                    e = O::add(e, u);
-                    u = O::add(d, O::mul(k.alpha, u));
+            bool ok = false;
+            if (i < n) {
+                R u = RealOps<R>::u01(kOO, st[s0 + i]);
+                R e = RealOps<R>::u01(kOO, st[s0 + n + i]);
+                R xv;
+                if constexpr (ALG == 0) {
+                    e = O::mul(static_cast<R>(-1), O::log(e));
+                    if (u > d) {
+                        const R t = O::mul(c, O::sub(static_cast<R>(1), u));
+                        u = -O::log(t);
+                        e = O::add(e, u);
+                        u = O::add(d, O::mul(k.alpha, u));
+                    }
+                    xv = O::exp(O::mul(c, O::log(u)));
+                    ok = fabs(xv) < e;
+                } else {
+                    u = O::mul(static_cast<R>(-1), O::log(u));
+                    e = O::mul(static_cast<R>(-1), O::log(e));
+                    xv = O::exp(O::mul(c, O::log(u)));
+                    u = O::add(u, e);
+                    e = O::add(d, xv);
+                    ok = u > e;
                 }
-                R xv = O::exp(O::mul(c, O::log(u)));
-                const R ua = fabs(xv);
-                x[j] = O::mul(beta, xv);
-                acc[j] = ua < e;
-            } else {
-                u = O::mul(static_cast<R>(-1), O::log(u));
-                e = O::mul(static_cast<R>(-1), O::log(e));
-                const R xv = O::exp(O::mul(c, O::log(u)));
-                u = O::add(u, e);
-                e = O::add(d, xv);
-                x[j] = O::mul(beta, xv);
-                acc[j] = u > e;
+                buf[i] = O::mul(beta, xv);
             }
+            const uint32_t m = __ballot_sync(0xffffffffu, ok);
+            if (lane == 0) fl.acc[warp + NW * j] = m;
         }
-        __syncthreads();
+        eng.batch(2ull * n, K, M);
+        pos += nw;
     } else {
         // ---- algorithm N: the batch normals, one Box-Muller pair per thread
-        // and pass into shared memory, then per element u, w, v = fma(c, w, 1)
-        R *wbuf = reinterpret_cast<R *>(smem + S::kMainBytes);
+        // and pass into shared memory
         const uint32_t nu = n / 2;
         const uint64_t q0 = s0 + n;  // first normal word in the staging buffer
+#pragma unroll 1
         for (uint32_t p = threadIdx.x; p < nu; p += THREADS) {
             const R u1 = RealOps<R>::u01(kOC, st[q0 + p]);
             const R u2 = O::mul(O::kTwoPi, RealOps<R>::u01(kOC, st[q0 + nu + p]));
             const R sr = O::sqrt(O::mul(static_cast<R>(-2), O::log(u1)));
             R sn, cs;
             O::sincos(u2, &sn, &cs);
-            wbuf[p] = O::mul(sr, sn);
-            wbuf[nu + p] = O::mul(sr, cs);
+            buf[p] = O::mul(sr, sn);
+            buf[nu + p] = O::mul(sr, cs);
         }
         if ((n & 1u) && threadIdx.x == THREADS - 1) {
             // odd n: the last normal from the two words after the batch
@@ -552,38 +552,27 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
             const R sr = O::mul(static_cast<R>(1), O::sqrt(O::mul(static_cast<R>(-2), O::log(a))));
             R sn, cs;
             O::sincos(O::mul(O::kTwoPi, b), &sn, &cs);
-            wbuf[n - 1] = O::add(static_cast<R>(0), O::mul(sr, cs));
+            buf[n - 1] = O::add(static_cast<R>(0), O::mul(sr, cs));
         }
         __syncthreads();
-        R u[EPT], w[EPT], v[EPT];
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
+        // ---- redraws of v = 1 + c w <= 0, in index order, by one warp
+        bool any = false;
+#pragma unroll 1
+        for (uint32_t j = 0; j < rounds; ++j) {
             const uint32_t i = threadIdx.x + j * THREADS;
-            u[j] = w[j] = v[j] = 0;
-            if (i >= n) continue;
-            u[j] = RealOps<R>::u01(kOO, st[s0 + i]);
-            w[j] = wbuf[i];
-            v[j] = O::fma(c, w[j], static_cast<R>(1));
+            const uint32_t m = __ballot_sync(0xffffffffu, i < n && O::fma(c, buf[i], static_cast<R>(1)) <= 0);
+            if (lane == 0) fl.red[warp + NW * j] = m;
+            any |= m != 0;
         }
-        // ---- redraws of v <= 0, in index order, by one thread
-        uint32_t *lidx = reinterpret_cast<uint32_t *>(smem);
-        R *lw = reinterpret_cast<R *>(smem + K * 4);
-        R *lv = lw + K;
-        int rk[EPT];
-        uint32_t nred = 0;
-        {
-            bool f[EPT];
-            uint32_t r[EPT];
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) f[j] = threadIdx.x + j * THREADS < n && v[j] <= 0;
-            block_rank_multi<THREADS, EPT>(f, shr, r, &nred);  // syncs: staging reads are done
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) {
-                rk[j] = f[j] ? static_cast<int>(r[j]) : -1;
-                if (f[j]) lidx[r[j]] = threadIdx.x + j * THREADS;
+        uint64_t nscalar = 0;
+        if (__syncthreads_or(any)) {
+            uint16_t *lidx = reinterpret_cast<uint16_t *>(smem + S::kRedrawAt);
+            mask_prefix(fl.red, fl.pre, rounds * NW);
+            const uint32_t nred = fl.pre[rounds * NW];
+            for (uint32_t j = 0; j < rounds; ++j) {
+                const uint32_t q = warp + NW * j, m = fl.red[q];
+                if ((m >> lane) & 1u) lidx[fl.pre[q] + __popc(m & lt)] = static_cast<uint16_t>(32 * q + lane);
             }
-        }
-        if (nred) {
             __syncthreads();
             if (threadIdx.x < 32) {
                 // The scalar normals after the batch words form one sequence
@@ -591,17 +580,15 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
                 // = r sin, the second returned from the cache); the q-th
                 // redrawn element takes the q-th z with 1 + c z > 0.  A warp
                 // evaluates 64 z at a time and assigns them by ballot ranks.
-                const int lane = threadIdx.x;
-                const unsigned lt = (1u << lane) - 1u;
                 ScalarWords<G, W> sw{&g, B, off};
                 const uint64_t sp0 = pos + nw;
                 uint32_t done = 0;
                 uint64_t used = 0;  // normals consumed
                 for (uint64_t pb = 0; done < nred; pb += 32) {
                     const uint64_t j = pb + lane;
-                    uint64_t k = sp0 + 2 * j;
+                    uint64_t kk = sp0 + 2 * j;
                     ScalarNormal<R> rn;
-                    const R z0 = rn(sw, k), z1 = rn(sw, k);
+                    const R z0 = rn(sw, kk), z1 = rn(sw, kk);
                     const R v0 = O::add(static_cast<R>(1), O::mul(c, z0));
                     const R v1 = O::add(static_cast<R>(1), O::mul(c, z1));
                     const bool a0 = v0 > 0, a1 = v1 > 0;
@@ -609,14 +596,8 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
                     const uint32_t before = __popc(m0 & lt) + __popc(m1 & lt);
                     const uint32_t r0 = before, r1 = before + (a0 ? 1u : 0u);
                     const uint32_t need = nred - done;
-                    if (a0 && r0 < need) {
-                        lw[done + r0] = z0;
-                        lv[done + r0] = v0;
-                    }
-                    if (a1 && r1 < need) {
-                        lw[done + r1] = z1;
-                        lv[done + r1] = v1;
-                    }
+                    if (a0 && r0 < need) buf[lidx[done + r0]] = z0;
+                    if (a1 && r1 < need) buf[lidx[done + r1]] = z1;
                     const uint32_t tot = __popc(m0) + __popc(m1);
                     if (tot >= need) {
                         // the need-th accepted normal is the last one consumed
@@ -633,40 +614,53 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
                 }
                 // consumed words: two per started pair (a cached second value
                 // is dropped with the chunk's normal generator)
-                if (lane == 0) *sh_pos = 2 * ((used + 1) / 2);
+                if (lane == 0) fl.words = 2 * ((used + 1) / 2);
             }
             __syncthreads();
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) {
-                if (rk[j] >= 0) {
-                    w[j] = lw[rk[j]];
-                    v[j] = lv[rk[j]];
-                }
-            }
+            nscalar = fl.words;
         }
-        const uint64_t nscalar = nred ? *sh_pos : 0;
+        // ---- acceptance.  v of a redrawn normal is rounded twice, of a batch
+        // normal once, as the two places of the reference do.
         const R db = O::mul(d, beta);
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            const uint32_t i = threadIdx.x + j * THREADS;
-            acc[j] = false;
-            if (i >= n) continue;
-            R e = O::mul(v[j], v[j]);
-            const R vv = O::mul(v[j], e);
-            e = O::mul(w[j], w[j]);
-            e = O::mul(e, e);
-            e = O::fma(-O::k0331, e, static_cast<R>(1));
-            x[j] = O::mul(db, vv);
-            if (u[j] < e) {
-                acc[j] = true;
-            } else {
-                const R a = O::mul(O::mul(w[j], w[j]), static_cast<R>(0.5));
+        auto v_of = [&](uint32_t i, R w) {
+            return (fl.red[i >> 5] >> (i & 31u)) & 1u ? O::add(static_cast<R>(1), O::mul(c, w))
+                                                      : O::fma(c, w, static_cast<R>(1));
+        };
+        uint16_t *list = fl.slow[warp];
+        uint32_t cnt = 0;
+        auto work_off = [&](uint32_t q) {  // the list's last q <= 32 values
+            __syncwarp();
+            cnt -= q;
+            if (lane < q) {
+                const uint32_t i = list[cnt + lane];
+                const R w = buf[i], v = v_of(i, w), vv = O::mul(v, O::mul(v, v));
+                const R a = O::mul(O::mul(w, w), static_cast<R>(0.5));
                 const R b = O::add(O::sub(static_cast<R>(1), vv), O::log(vv));
-                e = O::add(a, O::mul(d, b));
-                acc[j] = O::log(u[j]) < e;
+                buf[i] = O::mul(db, vv);
+                if (O::log(RealOps<R>::u01(kOO, st[s0 + i])) < O::add(a, O::mul(d, b)))
+                    atomicOr(&fl.acc[i >> 5], 1u << (i & 31u));
             }
+            __syncwarp();
+        };
+#pragma unroll 1
+        for (uint32_t j = 0; j < rounds; ++j) {
+            const uint32_t i = threadIdx.x + j * THREADS;
+            bool ok = false;
+            if (i < n) {
+                const R w = buf[i], v = v_of(i, w), vv = O::mul(v, O::mul(v, v));
+                R e = O::mul(w, w);
+                e = O::mul(e, e);
+                e = O::fma(-O::k0331, e, static_cast<R>(1));
+                ok = RealOps<R>::u01(kOO, st[s0 + i]) < e;
+                if (ok) buf[i] = O::mul(db, vv);
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, ok), sl = __ballot_sync(0xffffffffu, i < n && !ok);
+            if (lane == 0) fl.acc[warp + NW * j] = m;
+            if (i < n && !ok) list[cnt + __popc(sl & lt)] = static_cast<uint16_t>(i);
+            cnt += __popc(sl);
+            if (cnt >= 32) work_off(32);
         }
-        __syncthreads();  // every thread has read nscalar
+        if (cnt) work_off(cnt);
         // engine calls of the N chunk: uniforms, normals (+2 odd words), redraw words
         eng.batch(n, K, M);
         if (n == static_cast<uint32_t>(K)) {
@@ -683,37 +677,76 @@ __device__ uint32_t gamma_chunk(const G &g, const GammaParam<R> &k, const Ctr &B
         for (uint64_t q = 0; q < nscalar; ++q) eng.call(1, M);
         pos += nw + nscalar;
     }
-    if constexpr (ALG != 2) {
-        eng.batch(ALG <= 1 ? 2ull * n : n, K, M);
-        pos += nw;
-    }
-    if constexpr (ALG == 3) return got;
     // ---- compaction of the accepted values, in index order
-    uint32_t m = 0, r[EPT];
-    block_rank_multi<THREADS, EPT>(acc, shr, r, &m);
-#pragma unroll
-    for (int j = 0; j < EPT; ++j)
-        if (acc[j]) out[r[j]] = x[j];
-    return m;
+    mask_prefix(fl.acc, fl.pre, rounds * NW);
+    for (uint32_t j = 0; j < rounds; ++j) {
+        const uint32_t q = warp + NW * j, m = fl.acc[q];
+        if ((m >> lane) & 1u) out[fl.pre[q] + __popc(m & lt)] = buf[32 * q + lane];
+    }
+    return fl.pre[rounds * NW];
 }
 
-// gamma_distribution (:277-302) for `nstreams` streams of n values, all of
-// them drawn by algorithm ALG (one instantiation per algorithm keeps the code
-// each SM runs small).  Stream list[i] (i when list is null) writes
-// r + s * n; its engine starts at (ctr0 with word 1 = s, empty buffer) when
-// `blocks` is set, else at the engine state given (one stream), whose final
-// state goes to *ctr_out / *idx_out.
-constexpr int kGammaThreads = 256;
-
+// gamma_distribution (:277-302) of one stream of n values by algorithm ALG.
 template <class G, typename W, typename R, int THREADS, int ALG>
-__global__ void __launch_bounds__(THREADS, 3) k_gamma(G g, Ctr ctr0, uint32_t idx0, int blocks, uint64_t nstreams,
-    const uint32_t *list, uint64_t n, const GammaParam<R> *params, R *r, Ctr *ctr_out, uint32_t *idx_out)
+__device__ __forceinline__ void gamma_stream(const G &g, const GammaParam<R> &k, DevEngine<G::kCtrWords> &eng,
+    uint64_t n, R *o, unsigned char *smem, GammaFlags<THREADS, GammaTraits<R>::K> &fl)
 {
     using S = GammaSmem<G, W, R>;
     constexpr int K = S::K;
     constexpr uint32_t M = static_cast<uint32_t>(S::WPB);
-    __shared__ uint32_t shr[THREADS / 32 * GammaTraits<float>::K / THREADS + 1];
-    __shared__ uint64_t sh_pos;
+    // first word of the stream
+    Ctr B = eng.ctr;
+    uint32_t off = eng.idx;
+    if (eng.idx >= M) {
+        B = ctr_add(eng.ctr, 1, G::kCtrWords);
+        off = 0;
+    }
+    uint64_t pos = 0, left = n;
+    // chunks of K while more than K values are missing, then one of what is left
+    bool last;
+    uint32_t m;
+    do {
+        last = left <= static_cast<uint64_t>(K);
+        m = gamma_chunk<G, W, R, THREADS, ALG>(g, k, B, off, pos, eng,
+            last ? static_cast<uint32_t>(left) : static_cast<uint32_t>(K), o, smem, fl);
+        left -= m;
+        o += m;
+    } while (!last && m != 0);
+    if (left && threadIdx.x < 32) {
+        ScalarWords<G, W> sw{&g, B, off};
+        uint64_t end;
+        if constexpr (ALG != 2) {
+            end = pos + gamma_scalar_warp<R, ALG>(k, sw, pos, left, o);
+        } else {
+            end = gamma_scalar_n_warp<R, G>(k, sw, pos, left, o);
+        }
+        if (threadIdx.x == 0)
+            for (uint64_t q = pos; q < end; ++q) eng.call(1, M);
+    }
+}
+
+// One CTA per stream.  Stream list[i] (i when list is null) writes r + s n; its
+// engine starts at (ctr0 with word 1 = s, empty buffer) when `blocks` is set,
+// else at the engine state given (one stream), whose final state goes to
+// *ctr_out / *idx_out.  All algorithms are one launch, the list holding the
+// streams that take longest alone first, so the few streams of one algorithm
+// share the chip with the others' instead of running on a part of it before them.
+//
+// 4096 streams of 4096 values (Threefry, single precision, shapes 0.1 to 10): 32
+// + 54 + 317 us in a launch per algorithm with unrolled loops; the whole call 442
+// us then, 282 to 292 now.
+//
+// A call of one stream runs on one SM, chunk after chunk, and takes 1024 threads
+// there (100,000 values, Threefry, single precision, shapes 0.3 / 2.5: 445 / 432 us
+// with 256 threads and unrolled loops, 317 / 315 now).
+constexpr int kGammaThreads = 256, kGammaOneThreads = 1024;
+
+template <class G, typename W, typename R, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_gamma(G g, Ctr ctr0, uint32_t idx0, int blocks, uint64_t nstreams,
+    const uint32_t *list, uint64_t n, const GammaParam<R> *params, R *r, Ctr *ctr_out, uint32_t *idx_out)
+{
+    constexpr uint32_t M = static_cast<uint32_t>(GammaSmem<G, W, R>::WPB);
+    __shared__ GammaFlags<THREADS, GammaTraits<R>::K> fl;
     extern __shared__ __align__(16) unsigned char gamma_dyn[];
     g.prepare();
     unsigned char *smem = gamma_dyn + G::kDynSmem;
@@ -729,39 +762,12 @@ __global__ void __launch_bounds__(THREADS, 3) k_gamma(G g, Ctr ctr0, uint32_t id
             eng.ctr.w[2] = eng.ctr.w[3] = 0;
             eng.idx = M;
         }
-        // first word of the stream
-        Ctr B = eng.ctr;
-        uint32_t off = eng.idx;
-        if (eng.idx >= M) {
-            B = ctr_add(eng.ctr, 1, G::kCtrWords);
-            off = 0;
-        }
-        uint64_t pos = 0, left = n;
         R *o = r + sidx * n;
-        while (left > static_cast<uint64_t>(K)) {
-            const uint32_t m = gamma_chunk<G, W, R, THREADS, ALG>(g, k, B, off, pos, eng, K, o, smem, shr, &sh_pos);
-            if (m == 0) break;
-            left -= m;
-            o += m;
-        }
-        const uint32_t m = gamma_chunk<G, W, R, THREADS, ALG>(g, k, B, off, pos, eng, static_cast<uint32_t>(left), o,
-            smem, shr, &sh_pos);
-        left -= m;
-        o += m;
-        if constexpr (ALG != 2) {
-            if (left && threadIdx.x < 32) {
-                ScalarWords<G, W> sw{&g, B, off};
-                const uint64_t used = gamma_scalar_warp<R, ALG>(k, sw, pos, left, o);
-                if (threadIdx.x == 0)
-                    for (uint64_t q = 0; q < used; ++q) eng.call(1, M);
-            }
-        } else {
-            if (left && threadIdx.x < 32) {
-                ScalarWords<G, W> sw{&g, B, off};
-                const uint64_t sp = gamma_scalar_n_warp<R, G>(k, sw, pos, left, o);
-                if (threadIdx.x == 0)
-                    for (uint64_t q = pos; q < sp; ++q) eng.call(1, M);
-            }
+        switch (k.alg) {
+            case 0: gamma_stream<G, W, R, THREADS, 0>(g, k, eng, n, o, smem, fl); break;
+            case 1: gamma_stream<G, W, R, THREADS, 1>(g, k, eng, n, o, smem, fl); break;
+            case 2: gamma_stream<G, W, R, THREADS, 2>(g, k, eng, n, o, smem, fl); break;
+            default: gamma_stream<G, W, R, THREADS, 3>(g, k, eng, n, o, smem, fl); break;
         }
         if (!blocks && threadIdx.x == 0) {
             *ctr_out = eng.ctr;
@@ -771,49 +777,11 @@ __global__ void __launch_bounds__(THREADS, 3) k_gamma(G g, Ctr ctr0, uint32_t id
     }
 }
 
-template <class G, typename W, typename R, int ALG>
-int launch_gamma(const G &g, const Ctr &c0, uint32_t idx0, bool blocks, uint64_t count, const uint32_t *list,
-    uint64_t n, const GammaParam<R> *dparams, R *r, Ctr *dctr, uint32_t *didx, cudaStream_t s)
-{
-    using S = GammaSmem<G, W, R>;
-    auto kern = k_gamma<G, W, R, kGammaThreads, ALG>;
-    const int dyn = G::kDynSmem + S::kBytes;
-    MB_CUDA(allow_dyn_smem(kern, dyn));
-    int per_sm = 0;
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kGammaThreads, dyn));
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t cap = static_cast<uint64_t>(std::max(1, per_sm)) * sms;
-    const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(count, cap)));
-    kern<<<grid, kGammaThreads, dyn, s>>>(g, c0, idx0, blocks ? 1 : 0, count, list, n, dparams, r, dctr, didx);
-    MB_LAUNCH_CHECK();
-    return MCKL_B200_OK;
-}
-
-template <class G, typename W, typename R>
-int launch_gamma_alg(int alg, const G &g, const Ctr &c0, uint32_t idx0, bool blocks, uint64_t count,
-    const uint32_t *list, uint64_t n, const GammaParam<R> *dparams, R *r, Ctr *dctr, uint32_t *didx, cudaStream_t s)
-{
-    switch (alg) {
-        case 0: return launch_gamma<G, W, R, 0>(g, c0, idx0, blocks, count, list, n, dparams, r, dctr, didx, s);
-        case 1: return launch_gamma<G, W, R, 1>(g, c0, idx0, blocks, count, list, n, dparams, r, dctr, didx, s);
-        case 2: return launch_gamma<G, W, R, 2>(g, c0, idx0, blocks, count, list, n, dparams, r, dctr, didx, s);
-        default: return launch_gamma<G, W, R, 3>(g, c0, idx0, blocks, count, list, n, dparams, r, dctr, didx, s);
-    }
-}
-
-// One launch per algorithm present: the streams of each algorithm are listed
-// (device copy) so every CTA runs one algorithm's code.
 template <typename R>
 int gamma_impl(mckl_b200_engine_t *e, bool blocks, size_t nstreams, size_t n, const GammaParam<R> *hparams,
     size_t nparams, R *r, void *stream)
 {
     cudaStream_t s = as_stream(stream);
-    std::vector<uint32_t> lists[4];
-    if (blocks) {
-        for (size_t i = 0; i < nstreams; ++i) lists[hparams[i].alg].push_back(static_cast<uint32_t>(i));
-    }
     const size_t pbytes = align256(nparams * sizeof(GammaParam<R>));
     const size_t lbytes = align256(blocks ? nstreams * 4 : 4);
     char *scr = static_cast<char *>(scratch(6, pbytes + lbytes + 256, s));
@@ -823,14 +791,14 @@ int gamma_impl(mckl_b200_engine_t *e, bool blocks, size_t nstreams, size_t n, co
     Ctr *dctr = reinterpret_cast<Ctr *>(scr + pbytes + lbytes);
     uint32_t *didx = reinterpret_cast<uint32_t *>(scr + pbytes + lbytes + sizeof(Ctr));
     MB_CUDA(cudaMemcpyAsync(dparams, hparams, nparams * sizeof(GammaParam<R>), cudaMemcpyHostToDevice, s));
-    std::vector<uint32_t> flat;
-    size_t first[4] = {0, 0, 0, 0};
+    std::vector<uint32_t> list;
     if (blocks) {
-        for (int a = 0; a < 4; ++a) {
-            first[a] = flat.size();
-            flat.insert(flat.end(), lists[a].begin(), lists[a].end());
+        list.reserve(nstreams);
+        for (int a : {1, 0, 2, 3}) {
+            for (size_t i = 0; i < nstreams; ++i)
+                if (hparams[i].alg == a) list.push_back(static_cast<uint32_t>(i));
         }
-        MB_CUDA(cudaMemcpyAsync(dlist, flat.data(), flat.size() * 4, cudaMemcpyHostToDevice, s));
+        MB_CUDA(cudaMemcpyAsync(dlist, list.data(), list.size() * 4, cudaMemcpyHostToDevice, s));
     }
     const Ctr c0 = ctr_of(*e);
     const uint32_t idx0 = e->index;
@@ -839,17 +807,18 @@ int gamma_impl(mckl_b200_engine_t *e, bool blocks, size_t nstreams, size_t n, co
         using G = decltype(g);
         auto run = [&](auto wtag) {
             using W = decltype(wtag);
-            if (!blocks) {
-                return launch_gamma_alg<G, W, R>(hparams[0].alg, g, c0, idx0, false, 1, nullptr, n, dparams, r, dctr,
-                    didx, s);
-            }
-            for (int a = 0; a < 4; ++a) {
-                if (lists[a].empty()) continue;
-                const int rc2 = launch_gamma_alg<G, W, R>(a, g, c0, idx0, true, lists[a].size(), dlist + first[a], n,
-                    dparams, r, dctr, didx, s);
-                if (rc2 != MCKL_B200_OK) return rc2;
-            }
-            return MCKL_B200_OK;
+            auto launch = [&](auto threads) {
+                constexpr int T = decltype(threads)::value;
+                auto kern = k_gamma<G, W, R, T>;
+                const int dyn = G::kDynSmem + GammaSmem<G, W, R>::kBytes;
+                MB_CUDA(allow_dyn_smem(kern, dyn));
+                kern<<<static_cast<unsigned>(std::min<uint64_t>(nstreams, 0x7fffffffu)), T, dyn, s>>>(g, c0, idx0,
+                    blocks ? 1 : 0, nstreams, blocks ? dlist : nullptr, n, dparams, r, dctr, didx);
+                MB_LAUNCH_CHECK();
+                return static_cast<int>(MCKL_B200_OK);
+            };
+            if (blocks) return launch(std::integral_constant<int, kGammaThreads>{});
+            return launch(std::integral_constant<int, kGammaOneThreads>{});
         };
         if (w64) return run(uint64_t{});
         return run(uint32_t{});
@@ -864,7 +833,7 @@ int gamma_impl(mckl_b200_engine_t *e, bool blocks, size_t nstreams, size_t n, co
         set_ctr(*e, hc);
         e->index = hi;
     } else {
-        // the host lists must outlive the asynchronous copies
+        // the host list must outlive the asynchronous copies
         MB_CUDA(cudaStreamSynchronize(s));
     }
     return MCKL_B200_OK;
