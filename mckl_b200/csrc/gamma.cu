@@ -14,14 +14,14 @@
 // threads: the chunk's words are staged in shared memory, every thread
 // transforms K / THREADS values, the N redraws are assigned in index order by
 // one warp (the scalar normals they consume form one sequence, evaluated 64 at
-// a time), and the accepted values are compacted with a CTA-wide rank.
+// a time), and the accepted values are compacted with CTA-wide ranks.
 // Independent streams (gamma_blocks: one stream per block of samples, each on
 // its own counter range) run one per CTA across the GPU.
 //
 // Math: double uses the correctly rounded double-double log/exp/sin/cos of
-// crmath.cuh; float evaluates log/exp/sin/cos in double and rounds once (a
-// correctly rounded float result except in double-rounding cases, about one
-// in 2^28).  Every multiply and add is an explicit _rn operation, fma only
+// crmath.cuh; float evaluates log/exp/sin/cos in double (crmathf.cuh) and rounds
+// once (a correctly rounded float result except in double-rounding cases, about
+// one in 2^28).  Every multiply and add is an explicit _rn operation, fma only
 // where the reference calls fma.
 #include <algorithm>
 #include <cmath>

@@ -5,11 +5,13 @@
 // ESS < N * threshold (ResampleEval, algorithm/resample.hpp:494-507) -> next.
 // Model noise comes from one sequential engine, as BackendSEQ's eval_range
 // does with rng_set[0] (smp/backend_seq.hpp:60-64); resampling uses the
-// particle's own engine (core/particle.hpp:364).  Every piece is the
-// bit-faithful kernel of its reference function; the loop itself runs on the
-// host and waits once per step for the ESS that decides the resampling, as
-// the reference's loop does, with the next step's model noise (which does not
-// depend on the decision) already queued behind the read-back.
+// particle's own engine (core/particle.hpp:364).  A cloud that fits the chip's
+// shared memory (smc_coop.cu) runs its steps, decisions included, in cooperative
+// kernels.  For larger ones every piece is the kernel of its reference function
+// and the loop runs on the host, which waits once per step for the ESS that
+// decides the resampling, as the reference's loop does, with the next step's
+// model noise (which does not depend on the decision) already queued behind the
+// read-back.
 #include <algorithm>
 #include <cmath>
 #include <vector>

@@ -2,7 +2,9 @@
 // with uneven particle counts in one persistent kernel.
 //
 // Each CTA pulls filters from a work queue (largest first) and runs all T
-// steps of a filter before taking the next.  Per step and filter:
+// steps of a filter before taking the next; where the largest filters would
+// outlast the rest, clusters of four CTAs take them (pf_batched_joint.cu).  Per
+// step and filter:
 //   noise      Normal(0,1) from the filter's model stream, consumed exactly as
 //              normal_distribution does (random/normal_distribution.hpp:50-101:
 //              1024-value chunks, radius word i and angle word K/2 + i, odd n

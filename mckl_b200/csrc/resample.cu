@@ -17,6 +17,8 @@
 //     slots, in ascending order, take the surplus copies in source order.  A
 //     single-pass decoupled-look-back scan counts empties and surplus copies,
 //     each empty slot then finds its source by binary search.
+// Counts whose cloud fits the chip's shared memory come from one cooperative
+// kernel (smc_coop.cu); the kernels here serve larger clouds.
 #include <algorithm>
 
 #include "block_scan.cuh"

@@ -2,12 +2,15 @@
 //
 // Every kernel is a pure function of (generator key, first block counter,
 // word offset): thread i of the grid computes its blocks straight from the
-// counter, so there is no inter-thread dependency and no read traffic.  Two
+// counter, so there is no inter-thread dependency and no read traffic.  Three
 // shapes cover every call:
 //   * aligned: the stream starts on a block boundary and the output is
-//     16-byte aligned -> each thread turns whole blocks into 128-bit stores;
-//   * staged: any start offset / alignment -> a CTA generates a tile of blocks
-//     into shared memory and writes its outputs from there, coalesced.
+//     16-byte aligned -> each thread turns whole blocks into 128-bit stores,
+//     the values of a last partial block in the same launch;
+//   * shifted: 4096 values or more from the middle of a block into a 16-byte
+//     aligned output -> the same stores, the values shifted between lanes;
+//   * staged: short calls and other alignments -> a CTA generates a tile of
+//     blocks into shared memory and writes its outputs from there, coalesced.
 // The Normal transform pairs the two halves of each 8192-byte chunk
 // (random/normal_distribution.hpp:50-78), so one CTA owns one chunk and stages
 // the chunk's words in shared memory.

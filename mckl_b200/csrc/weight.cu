@@ -11,6 +11,8 @@
 // fold (fold.cuh); the per-chunk dot products are short independent folds,
 // one thread each.  The log of the normalising-constant ratio
 // log sum_i W_i^old exp(v_i) = lmax + log(accw) is returned alongside.
+// Arrays that fit the chip's shared memory take one cooperative kernel
+// (smc_coop.cu); the kernels here serve larger ones.
 #include <algorithm>
 
 #include "block_scan.cuh"
