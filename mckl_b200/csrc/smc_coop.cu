@@ -20,7 +20,7 @@ __device__ __forceinline__ Ctx make_ctx(Shared &sh, const Global &g, unsigned T)
     // no CTA stores into another's shared memory before that one runs
     if (cluster)
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    return Ctx{g, &sh, T, blockIdx.x, 0, 0, 0, cluster};
+    return Ctx{g, &sh, T, blockIdx.x, 0, 0, 0, 0, cluster};
 }
 
 // A tile's dynamic shared memory: its values and its 64-bit integers, padded.
@@ -354,7 +354,7 @@ Tiling tiling(uint64_t n)
 // bytes; the slots are cleared on the stream when there are exchanges.
 int coop_scratch(const Tiling &t, uint64_t n, size_t extra, Global *g, CoopResult **res, char **more, cudaStream_t s)
 {
-    const size_t win = t.T > 1 ? align256(static_cast<size_t>(t.T) * kTileWin * sizeof(Window)) : 0;
+    const size_t win = t.T > 1 ? align256(static_cast<size_t>(kWinSets) * t.T * kTileWin * sizeof(Window)) : 0;
     const size_t dots = align256((n + 1023) / 1024 * sizeof(double));
     char *p = static_cast<char *>(scratch(9, kHeader + align256(kSlotBytes) + win + dots + extra, s));
     if (!p) {

@@ -42,6 +42,7 @@ constexpr int kMaxWarps = 32;
 constexpr unsigned kMaxTiles = 148;   // one CTA per SM
 constexpr unsigned kMaxTile = 8192;   // elements
 constexpr unsigned kTileWin = 256;    // windows a tile can list
+constexpr unsigned kWinSets = 2;      // sets of window lists: folds take them in turn (fold_grid)
 constexpr unsigned kWin = 512;        // windows of a fold the walk takes
 constexpr unsigned kSegWin = 64;      // windows of one short fold (seg_fold)
 constexpr unsigned kMaxCluster = 8;   // tiles that exchange through distributed shared memory
@@ -58,7 +59,7 @@ struct Window {
 struct Global {
     ulonglong2 *slots;  // [2][kMaxVals][kMaxTiles]: {value, epoch}
     ulonglong2 *chain;  // [kMaxTiles]: {tile's last value, epoch} of the event-loop fold
-    Window *win;        // [tiles][kTileWin]
+    Window *win;        // [kWinSets][tiles][kTileWin]
     double *dots;       // [ceil(N / 1024)] chunk dot products
     int *err;           // set when a wait gave up
 };
@@ -94,6 +95,7 @@ struct Ctx {
     Shared *sh;
     uint32_t T, tile;
     unsigned long long epoch, chain_epoch;
+    unsigned folds;  // fold_grid calls so far, the same in every CTA
     unsigned flip;
     bool cluster;  // the T CTAs are one cluster
 };
@@ -669,12 +671,20 @@ __device__ __forceinline__ bool fold_approx(Ctx &c, const double *s_v, Approx &a
 // and the one before the thread's first element goes to *before.  What was
 // written to global memory before the call is visible after it (its exchange
 // carries data).  s_q is overwritten.  False when a wait gave up.
+//
+// A tile writes its window list before the exchange and reads every tile's after
+// it, and the next fold may follow with no exchange between (resample_phase with
+// known sums).  So folds take two sets of lists in turn: a CTA that writes fold
+// n + 2's list is behind the exchange of fold n + 1, which every CTA enters only
+// after it has read the lists of fold n.  With one set a CTA that is ahead would
+// rewrite its list while another still reads it.
 template <int THR, int PER, bool PREFIX>
 __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint64_t n, const Approx ap,
     double *total, double *before)
 {
     Shared *sh = c.sh;
     const uint64_t i0 = (static_cast<uint64_t>(c.tile) * THR + threadIdx.x) * PER;
+    Window *lists = c.g.win + static_cast<size_t>(++c.folds % kWinSets) * c.T * kTileWin;
     if (threadIdx.x == 0) sh->elast = -1;
     __syncthreads();
     unsigned win;
@@ -697,7 +707,7 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
                     sh->wx[rk] = x;
                     sh->wP[rk] = Pk;
                 } else {
-                    c.g.win[static_cast<size_t>(c.tile) * kTileWin + rk] = Window{x, Pk, q};
+                    lists[static_cast<size_t>(c.tile) * kTileWin + rk] = Window{x, Pk, q};
                 }
                 ++rk;
             } else {
@@ -757,7 +767,7 @@ __device__ __noinline__ bool fold_grid(Ctx &c, double *s_v, long long *s_q, uint
                         hi = mid;
                     }
                 }
-                const Window *w = c.g.win + static_cast<size_t>(lo) * kTileWin + (k - sh->pw[lo]);
+                const Window *w = lists + static_cast<size_t>(lo) * kTileWin + (k - sh->pw[lo]);
                 sh->wx[k] = __ldcg(&w->x);
                 sh->wP[k] = sh->pq[lo] + __ldcg(&w->P);
                 sh->we[k] = static_cast<int>(__ldcg(&w->e));
