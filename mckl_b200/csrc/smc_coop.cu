@@ -137,7 +137,6 @@ struct FilterArgs {
     uint8_t *resampled;
     unsigned long long *ties;
     double *loglik;
-    int *last;  // which of xb holds the particles at the end
 };
 
 __device__ __noinline__ double log_rn(double x)
@@ -291,7 +290,7 @@ __global__ void __launch_bounds__(THR, 1) k_coop_filter(Global g, unsigned T, Fi
         flat = true;
         accw = 1.0;
     }
-    // the final weights; the particles stay in xb[cur]
+    // the final weights; the particles are in xb[cur], the caller's buffer
     const double inv = __ddiv_rn(1.0, accw);
 #pragma unroll 2
     for (int k = 0; k < PER; ++k) {
@@ -299,10 +298,7 @@ __global__ void __launch_bounds__(THR, 1) k_coop_filter(Global g, unsigned T, Fi
         if (base + o < N) a.W[base + o] = flat ? a.equal : __dmul_rn(inv, tm.v[pad(o)]);
     }
     if (ties) atomicAdd(a.ties, ties);
-    if (lead) {
-        *a.loglik = ll_sum;
-        *a.last = cur;
-    }
+    if (lead) *a.loglik = ll_sum;
 }
 
 // ---------------------------------------------------------------------------
@@ -471,8 +467,8 @@ int coop_filter(const CoopFilter &f, double *loglik, double *ess, uint8_t *resam
     const uint64_t N = f.N, T = f.T;
     const Tiling t = tiling(N);
     if (!t.T) return kCoopNo;
-    // results: loglik, ties, last, ess[T + 1], resampled[T + 1]
-    const size_t rbytes = align256(24 + (T + 1) * 9);
+    // results: loglik, ties, ess[T + 1], resampled[T + 1]
+    const size_t rbytes = align256(16 + (T + 1) * 9);
     const size_t tile_words = static_cast<size_t>(t.T) * t.threads * t.per;
     Global g;
     CoopResult *res;
@@ -489,9 +485,8 @@ int coop_filter(const CoopFilter &f, double *loglik, double *ess, uint8_t *resam
     char *rb = take(rbytes);
     a.loglik = reinterpret_cast<double *>(rb);
     a.ties = reinterpret_cast<unsigned long long *>(rb + 8);
-    a.last = reinterpret_cast<int *>(rb + 16);
-    a.ess = reinterpret_cast<double *>(rb + 24);
-    a.resampled = reinterpret_cast<uint8_t *>(rb + 24 + (T + 1) * 8);
+    a.ess = reinterpret_cast<double *>(rb + 16);
+    a.resampled = reinterpret_cast<uint8_t *>(rb + 16 + (T + 1) * 8);
     double *y = reinterpret_cast<double *>(take((T + 1) * 8));
     a.y = y;
     a.N = N;
@@ -508,14 +503,15 @@ int coop_filter(const CoopFilter &f, double *loglik, double *ess, uint8_t *resam
         a.rkey[k] = f.rkey[k];
     }
     a.scheme = f.scheme;
-    a.xb[0] = f.x;
-    a.xb[1] = reinterpret_cast<double *>(take(N * 8));
+    // the buffers change at each of the T steps: the particles end in f.x
+    a.xb[T & 1] = f.x;
+    a.xb[(T & 1) ^ 1] = reinterpret_cast<double *>(take(N * 8));
     a.W = f.W;
     a.anc = f.anc;
     a.ubuf = reinterpret_cast<double *>(take(N * 8));
     a.surp = reinterpret_cast<uint32_t *>(take(tile_words * 4));
     MB_CUDA(cudaMemcpyAsync(y, f.y, (T + 1) * 8, cudaMemcpyHostToDevice, s));
-    MB_CUDA(cudaMemsetAsync(rb, 0, 24, s));
+    MB_CUDA(cudaMemsetAsync(rb, 0, 16, s));
     rc = COOP_LAUNCH(k_coop_filter, t, s, g, t.T, a);
     if (rc != MCKL_B200_OK) return rc;
     std::unique_ptr<char[]> h(new (std::nothrow) char[rbytes]);
@@ -533,10 +529,8 @@ int coop_filter(const CoopFilter &f, double *loglik, double *ess, uint8_t *resam
     };
     *loglik = word(0, 0.0);
     *ties = word(8, uint64_t{0});
-    if (ess) std::memcpy(ess, h.get() + 24, (T + 1) * 8);
-    if (resampled) std::memcpy(resampled, h.get() + 24 + (T + 1) * 8, T + 1);
-    if (word(16, int{0}))
-        MB_CUDA(cudaMemcpyAsync(f.x, a.xb[1], N * 8, cudaMemcpyDeviceToDevice, s));
+    if (ess) std::memcpy(ess, h.get() + 16, (T + 1) * 8);
+    if (resampled) std::memcpy(resampled, h.get() + 16 + (T + 1) * 8, T + 1);
     return MCKL_B200_OK;
 }
 
