@@ -72,6 +72,9 @@ uint64_t mckl_b200_launch_count(void);
  * than the stream's previous calls; growing is refused with
  * MCKL_B200_ERR_NOMEM while the stream is being captured into a CUDA graph,
  * so make one call of the largest size on a stream before capturing it.
+ * A kernel of such a call that gives up a wait between its CTAs sets an error
+ * word; a call that does not synchronize leaves it to the stream's next one
+ * that does, which returns MCKL_B200_ERR_DEVICE.
  * mckl_b200_release_stream frees the buffers held for `stream` on the current
  * device (after its queued work); call it before destroying a stream the
  * library has used.  No counterpart in the reference (its objects own their

@@ -94,7 +94,7 @@ void *scratch(int slot, size_t bytes, cudaStream_t stream)
             b.ptr = nullptr;
             return nullptr;
         }
-        // a new buffer's header is zero (the cooperative kernels keep an error word there)
+        // a new buffer's first bytes are zero (the cooperative kernels' error word)
         if (cudaMemsetAsync(b.ptr, 0, 256, stream) != cudaSuccess) {
             cudaFreeAsync(b.ptr, stream);
             b.ptr = nullptr;

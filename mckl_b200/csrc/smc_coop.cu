@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(THR, 1) k_coop_filter(Global g, unsigned T, Fi
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
-constexpr size_t kHeader = 256;  // CoopResult; zeroed when the buffer is allocated
+constexpr int kResultSlot = 9, kWorkSlot = 11;  // scratch() slots
 constexpr size_t kSlotBytes = (2 * kMaxVals + 1) * kMaxTiles * sizeof(ulonglong2);
 
 // CTAs of `kernel` that the current device holds at once (0 when it cannot
@@ -347,19 +347,20 @@ Tiling tiling(uint64_t n)
 }
 
 // Working memory of a launch of T tiles over n elements with `extra` more
-// bytes; the slots are cleared on the stream when there are exchanges.
+// bytes; the slots are cleared on the stream when there are exchanges.  The
+// results have a small buffer of their own, zeroed when it is allocated: it never
+// grows, so an error word that no call has read yet is kept.
 int coop_scratch(const Tiling &t, uint64_t n, size_t extra, Global *g, CoopResult **res, char **more, cudaStream_t s)
 {
     const size_t win = t.T > 1 ? align256(static_cast<size_t>(kWinSets) * t.T * kTileWin * sizeof(Window)) : 0;
     const size_t dots = align256((n + 1023) / 1024 * sizeof(double));
-    char *p = static_cast<char *>(scratch(9, kHeader + align256(kSlotBytes) + win + dots + extra, s));
-    if (!p) {
+    *res = static_cast<CoopResult *>(scratch(kResultSlot, sizeof(CoopResult), s));
+    char *p = static_cast<char *>(scratch(kWorkSlot, align256(kSlotBytes) + win + dots + extra, s));
+    if (!*res || !p) {
         set_error("scratch allocation failed");
         return MCKL_B200_ERR_NOMEM;
     }
-    *res = reinterpret_cast<CoopResult *>(p);
     g->err = &(*res)->err;
-    p += kHeader;
     g->slots = reinterpret_cast<ulonglong2 *>(p);
     g->chain = g->slots + 2 * kMaxVals * kMaxTiles;
     if (t.T > 1) MB_CUDA(cudaMemsetAsync(p, 0, kSlotBytes, s));

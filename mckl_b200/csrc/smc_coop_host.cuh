@@ -13,7 +13,8 @@ namespace mckl_b200 {
 constexpr int kCoopNo = 1;
 
 // Results of a call, in device memory of the stream's (CoopResult *res).
-// err stays set until a call has reported it (coop_read).
+// err stays set until a call has reported it (coop_read): a wait that gave up in a
+// call that does not synchronize is reported by the stream's next one that does.
 struct CoopResult {
     int err, pad;
     double ess, log_nc, accw, lmax;
