@@ -66,8 +66,10 @@ uint64_t mckl_b200_launch_count(void);
 /* Working memory.  Calls that need device working memory beyond their
  * arguments (Weight, fold, resampling, rep -> index, the plain filter, Gamma,
  * the index matrix, the weighted estimate) take it from buffers the library
- * keeps per (device, stream): calls on different streams or host threads
- * never share them, calls on one stream are ordered by it.  A buffer grows
+ * keeps per (device, stream) and kind of call: calls on different streams
+ * never share them, calls on one stream are ordered by it.  Host threads that
+ * use one stream may make different calls at the same time; two calls of one
+ * kind on one stream must not be queued at the same time.  A buffer grows
  * (stream-ordered, without synchronising the device) when a call needs more
  * than the stream's previous calls; growing is refused with
  * MCKL_B200_ERR_NOMEM while the stream is being captured into a CUDA graph,

@@ -304,7 +304,11 @@ __global__ void __launch_bounds__(THR, 1) k_coop_filter(Global g, unsigned T, Fi
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
-constexpr int kResultSlot = 9, kWorkSlot = 11;  // scratch() slots
+// scratch() slots: the results, and the working memory of each kind of call.  A
+// launch's exchange slots are cleared before it, and all launches count epochs
+// from 1, so between a call's clear and its launch no other may use the slots:
+// two host threads that make different calls on one stream share none.
+constexpr int kResultSlot = 9, kWeightSlot = 11, kResampleSlot = 12, kIndexSlot = 13, kFilterSlot = 14;
 constexpr size_t kSlotBytes = (2 * kMaxVals + 1) * kMaxTiles * sizeof(ulonglong2);
 
 // CTAs of `kernel` that the current device holds at once (0 when it cannot
@@ -346,16 +350,17 @@ Tiling tiling(uint64_t n)
     return {0, 0, 0};
 }
 
-// Working memory of a launch of T tiles over n elements with `extra` more
-// bytes; the slots are cleared on the stream when there are exchanges.  The
+// Working memory (buffer `slot`) of a launch of T tiles over n elements with
+// `extra` more bytes; the slots are cleared on the stream when there are exchanges.  The
 // results have a small buffer of their own, zeroed when it is allocated: it never
 // grows, so an error word that no call has read yet is kept.
-int coop_scratch(const Tiling &t, uint64_t n, size_t extra, Global *g, CoopResult **res, char **more, cudaStream_t s)
+int coop_scratch(int slot, const Tiling &t, uint64_t n, size_t extra, Global *g, CoopResult **res, char **more,
+    cudaStream_t s)
 {
     const size_t win = t.T > 1 ? align256(static_cast<size_t>(kWinSets) * t.T * kTileWin * sizeof(Window)) : 0;
     const size_t dots = align256((n + 1023) / 1024 * sizeof(double));
     *res = static_cast<CoopResult *>(scratch(kResultSlot, sizeof(CoopResult), s));
-    char *p = static_cast<char *>(scratch(kWorkSlot, align256(kSlotBytes) + win + dots + extra, s));
+    char *p = static_cast<char *>(scratch(slot, align256(kSlotBytes) + win + dots + extra, s));
     if (!*res || !p) {
         set_error("scratch allocation failed");
         return MCKL_B200_ERR_NOMEM;
@@ -430,7 +435,7 @@ int coop_weight(uint64_t N, double *W, const double *v, int add_log, CoopResult 
     if (!t.T) return kCoopNo;
     Global g;
     char *more;
-    const int rc = coop_scratch(t, N, 0, &g, res, &more, s);
+    const int rc = coop_scratch(kWeightSlot, t, N, 0, &g, res, &more, s);
     if (rc != MCKL_B200_OK) return rc;
     return COOP_LAUNCH(k_coop_weight, t, s, g, t.T, N, W, v, add_log, *res);
 }
@@ -443,7 +448,7 @@ int coop_resample(int scheme, uint64_t N, uint64_t M, const double *W, const dou
     if (!t.T) return kCoopNo;
     Global g;
     char *more;
-    const int rc = coop_scratch(t, n, align256(n * sizeof(double)), &g, res, &more, s);
+    const int rc = coop_scratch(kResampleSlot, t, n, align256(n * sizeof(double)), &g, res, &more, s);
     if (rc != MCKL_B200_OK) return rc;
     return COOP_LAUNCH(k_coop_resample, t, s, g, t.T, scheme, N, M, W, canon, reinterpret_cast<double *>(more), rep,
         *res);
@@ -456,8 +461,8 @@ int coop_rep_to_index(uint64_t N, uint64_t M, const uint64_t *rep, uint64_t *idx
     if (!t.T) return kCoopNo;
     Global g;
     char *more;
-    const int rc = coop_scratch(t, n, align256(static_cast<size_t>(t.T) * t.threads * t.per * sizeof(uint32_t)), &g, res, &more,
-        s);
+    const int rc = coop_scratch(kIndexSlot, t, n, align256(static_cast<size_t>(t.T) * t.threads * t.per * sizeof(uint32_t)),
+        &g, res, &more, s);
     if (rc != MCKL_B200_OK) return rc;
     if (t.T == 1) *res = nullptr;
     return COOP_LAUNCH(k_coop_index, t, s, g, t.T, N, M, rep, reinterpret_cast<uint32_t *>(more), idx);
@@ -474,8 +479,8 @@ int coop_filter(const CoopFilter &f, double *loglik, double *ess, uint8_t *resam
     Global g;
     CoopResult *res;
     char *p;
-    int rc = coop_scratch(t, N, rbytes + align256((T + 1) * 8) + 2 * align256(N * 8) + align256(tile_words * 4), &g, &res,
-        &p, s);
+    int rc = coop_scratch(kFilterSlot, t, N,
+        rbytes + align256((T + 1) * 8) + 2 * align256(N * 8) + align256(tile_words * 4), &g, &res, &p, s);
     if (rc != MCKL_B200_OK) return rc;
     auto take = [&p](size_t n) {
         char *q = p;
