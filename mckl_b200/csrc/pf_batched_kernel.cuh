@@ -1101,9 +1101,21 @@ struct FilterRun {
         for (uint32_t u = u0; u < uend; u += THREADS) {
             const float4 a = jt.e[2 * u], b = jt.e[2 * u + 1];
             jt.sc[u] = meet(fmax(fmax(fmax(a.x, a.y), fmax(a.z, a.w)), fmax(fmax(b.x, b.y), fmax(b.z, b.w))));
+            // minus infinity (a weight of zero, or an unused slot) is a term of zero
             const auto ex = [m](R v) { return v == -INFINITY ? R(0) : O::exp(O::sub(v, m)); };
             jt.e[2 * u] = make_float4(ex(a.x), ex(a.y), ex(a.z), ex(a.w));
             jt.e[2 * u + 1] = make_float4(ex(b.x), ex(b.y), ex(b.z), ex(b.w));
+            // except that step()'s terms are not numbers while the running maximum is
+            // minus infinity
+            if (m == -INFINITY) {
+                uint32_t pa[4], pb[4];
+                uint64_t src;
+                int lo, hi;
+                lay.slots(t, u, pa, pb, &lo, &hi, &src);
+                R *e = reinterpret_cast<R *>(jt.e + 2 * u);
+#pragma unroll 1
+                for (int k = 2 * lo; k < 2 * hi; ++k) e[k] = O::sub(m, m);
+            }
         }
         if (odd) {
             jt.sc[units] = meet(vodd);
