@@ -275,15 +275,23 @@ int mckl_b200_batched_shadow_params(mckl_b200_batched_t *b, const double *phi, c
 /* Adjoint: the gradient of each filter's FP64 log-likelihood estimate with
  * respect to (phi, sx, sy), resampling times and ancestor indices held fixed
  * (no counterpart in the reference, which has no derivatives).  The forward
- * pass keeps a checkpoint every `checkpoint_every` steps; the backward pass
- * replays each block of steps from its checkpoint -- the noise, decisions and
- * ancestors are recomputed from the counters, not stored -- and sweeps it in
+ * pass keeps a checkpoint every C = min(checkpoint_every, T) steps; the
+ * backward pass replays each block of steps from its checkpoint -- the noise,
+ * decisions and ancestors are recomputed from the counters -- and sweeps it in
  * reverse.  Handle created with fp64 = 1.  loglik: F doubles (may be NULL),
  * grad: F x 3 doubles (d/dphi, d/dsx, d/dsy), both HOST arrays; synchronizes
- * `stream`.  Device memory: checkpoints 16 B x particles x (T / C + 1) plus
- * per-SM replay records of C x the largest N x 28 B. */
+ * `stream`.  Device memory, kept by the handle: checkpoints of 16 B x
+ * particles x (T / C + 1), and for each CTA (one per filter, at most one per
+ * SM) replay records of C x the largest N x 28 B and vectors of the largest
+ * N x 24 B. */
 int mckl_b200_batched_adjoint(mckl_b200_batched_t *b, int checkpoint_every, double *loglik, double *grad,
                               void *stream);
+/* The same with leave to use more memory: when replay records of all T steps
+ * (CTAs x T x the largest N x 28 B) take no more than record_bytes, they are
+ * kept instead of checkpoints and the run is not repeated, with the same
+ * results.  record_bytes = 0 is mckl_b200_batched_adjoint. */
+int mckl_b200_batched_adjoint_records(mckl_b200_batched_t *b, int checkpoint_every, size_t record_bytes,
+                                      double *loglik, double *grad, void *stream);
 
 /* Score estimate by the Fisher identity (no counterpart in the reference):
  * grad log p(y_1:T | theta) = E[grad log p(x_0:T, y_1:T | theta) | y_1:T],

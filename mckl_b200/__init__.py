@@ -198,7 +198,7 @@ _bt_set_y = _bind("mckl_b200_batched_set_y", [_vp, _vp, _vp])
 _bt_autotune = _bind("mckl_b200_batched_autotune", [_vp, _i, _vp, _vp, _vp, _vp, _vp])
 _bt_get_config = _bind("mckl_b200_batched_get_config", [_vp, _vp, _vp])
 _bt_shadow_params = _bind("mckl_b200_batched_shadow_params", [_vp, _vp, _vp, _vp])
-_bt_adjoint = _bind("mckl_b200_batched_adjoint", [_vp, _i, _vp, _vp, _vp])
+_bt_adjoint = _bind("mckl_b200_batched_adjoint_records", [_vp, _i, _sz, _vp, _vp, _vp])
 _bt_score = _bind("mckl_b200_batched_score", [_vp, _vp, _vp, _vp])
 _bt_set_params = _bind("mckl_b200_batched_set_params", [_vp, _vp, _vp, _vp, _vp])
 _bt_set_keys = _bind("mckl_b200_batched_set_keys", [_vp, _vp, _vp, _vp])
@@ -213,6 +213,14 @@ _pmcmc_prop = _bind("mckl_b200_pmcmc_ar1_proposal", [_sz, _vp, _sz, _vp, _vp, _P
 
 def _arr(a, dt):
     return np.ascontiguousarray(a, dtype=dt)
+
+
+class _DefaultInterval(int):
+    """The adjoint's default interval, told apart from the same number given by a caller."""
+
+
+CHECKPOINT_EVERY = _DefaultInterval(32)
+ADJOINT_RECORD_BYTES = 4 << 30  # device memory that the default interval may use for whole-run records
 
 
 class BatchedFilters:
@@ -271,12 +279,17 @@ class BatchedFilters:
         a = [_arr(v, np.float64) for v in (phi, sx, sy)]
         _check(_bt_shadow_params(self.h, *[v.ctypes.data_as(ctypes.c_void_p) for v in a]))
 
-    def adjoint(self, checkpoint_every=32, stream=None):
+    def adjoint(self, checkpoint_every=CHECKPOINT_EVERY, stream=None):
         """(loglik[F], grad[F, 3]): the FP64 estimate and its gradient with
-        respect to (phi, sx, sy), ancestors held fixed (fp64=True handles)."""
+        respect to (phi, sx, sy), ancestors held fixed (fp64=True handles).
+        By default the records of the whole run are kept when they take no more
+        than ADJOINT_RECORD_BYTES, which is faster; an interval that is given
+        bounds the memory as mckl_b200_batched_adjoint states it.  The results
+        are the same."""
         ll = np.zeros(self.F)
         g = np.zeros((self.F, 3))
-        _check(_bt_adjoint(self.h, int(checkpoint_every), ll.ctypes.data_as(ctypes.c_void_p),
+        limit = ADJOINT_RECORD_BYTES if checkpoint_every is CHECKPOINT_EVERY else 0
+        _check(_bt_adjoint(self.h, int(checkpoint_every), limit, ll.ctypes.data_as(ctypes.c_void_p),
                            g.ctypes.data_as(ctypes.c_void_p), _stream_ptr(stream)))
         return ll, g
 

@@ -13,12 +13,12 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import BatchedFilters, _check, _bt_shadow_params  # noqa: F401
+from . import CHECKPOINT_EVERY, BatchedFilters, _check, _bt_shadow_params  # noqa: F401
 
 
 class PFLogLikelihood(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, phi, sx, sy, template: dict, checkpoint_every: int = 32):
+    def forward(ctx, phi, sx, sy, template: dict, checkpoint_every: int = CHECKPOINT_EVERY):
         w = dict(template)
         w["phi"] = phi.detach().cpu().double().numpy()
         w["sx"] = sx.detach().cpu().double().numpy()
@@ -43,7 +43,7 @@ class PFLogLikelihood(torch.autograd.Function):
         return gout * grad[:, 0], gout * grad[:, 1], gout * grad[:, 2], None, None
 
 
-def loglik(phi, sx, sy, workload: dict, checkpoint_every: int = 32):
+def loglik(phi, sx, sy, workload: dict, checkpoint_every: int = CHECKPOINT_EVERY):
     """Differentiable FP64 log-likelihood estimates of the workload's filters."""
     return PFLogLikelihood.apply(phi, sx, sy, workload, checkpoint_every)
 

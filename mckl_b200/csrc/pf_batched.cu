@@ -1069,6 +1069,12 @@ int mckl_b200_batched_set_keys(mckl_b200_batched_t *b, const uint32_t *mkeys, co
 int mckl_b200_batched_adjoint(mckl_b200_batched_t *b, int checkpoint_every, double *loglik, double *grad,
     void *stream)
 {
+    return mckl_b200_batched_adjoint_records(b, checkpoint_every, 0, loglik, grad, stream);
+}
+
+int mckl_b200_batched_adjoint_records(mckl_b200_batched_t *b, int checkpoint_every, size_t record_bytes,
+    double *loglik, double *grad, void *stream)
+{
     MB_CHECK_ARG(b != nullptr && grad != nullptr, "null argument");
     MB_CHECK_ARG(b->fp64 == 1 && b->a.xsa == nullptr, "the adjoint needs a handle created with fp64 = 1");
     MB_CHECK_ARG(checkpoint_every >= 1 && checkpoint_every <= 4096, "checkpoint_every in [1, 4096]");
@@ -1085,11 +1091,11 @@ int mckl_b200_batched_adjoint(mckl_b200_batched_t *b, int checkpoint_every, doub
                2 * align256(ctas * C * nm * 8) + 3 * align256(ctas * C * nm * 4) + align256(ctas * C) +
                align256(ctas * C * 4) + 3 * align256(ctas * nm * 8) + align256(static_cast<size_t>(b->F) * 24);
     };
-    // Records of the whole run, when they take no more than 4 GiB, replace the
+    // Records of the whole run, when the caller allows their memory, replace the
     // forward pass that the replay repeats: 256 filters x 8192 particles x 100
     // steps (3.4 GB of records) 24.4 -> 16.6 ms.
     uint64_t C = std::min<uint64_t>(static_cast<uint64_t>(checkpoint_every), T);
-    if (C < T && ctas * T * nm * 28 <= (4ull << 30)) C = T;
+    if (C < T && ctas * T * nm * 28 <= record_bytes) C = T;
     for (;;) {
         const size_t need = bytes_for(C);
         if (b->adj_bytes >= need) break;
