@@ -720,6 +720,7 @@ struct mckl_b200_batched {
     uint64_t nmax = 0;                         // largest particle count
     void *adj_mem = nullptr;                   // adjoint checkpoints and work areas
     size_t adj_bytes = 0;
+    size_t adj_refused = ~size_t{0};           // least size of whole-run records that could not be allocated
     void *score_mem = nullptr;                 // score estimator work areas
     size_t score_bytes = 0;
 };
@@ -1095,26 +1096,36 @@ int mckl_b200_batched_adjoint_records(mckl_b200_batched_t *b, int checkpoint_eve
     // forward pass that the replay repeats: 256 filters x 8192 particles x 100
     // steps (3.4 GB of records) 24.4 -> 16.6 ms.
     uint64_t C = std::min<uint64_t>(static_cast<uint64_t>(checkpoint_every), T);
-    if (C < T && ctas * T * nm * 28 <= record_bytes) C = T;
-    for (;;) {
-        const size_t need = bytes_for(C);
-        if (b->adj_bytes >= need) break;
+    if (C < T && ctas * T * nm * 28 <= record_bytes) {
+        // Their memory is taken before the handle's is given back, so a failure
+        // leaves what the checkpoints need; it is remembered, not tried again.
+        const size_t need = bytes_for(T);
+        void *m = nullptr;
+        if (b->adj_bytes < need && need < b->adj_refused) {
+            if (cudaMalloc(&m, need) == cudaSuccess) {
+                if (b->adj_mem) cudaFree(b->adj_mem);
+                b->adj_mem = m;
+                b->adj_bytes = need;
+            } else {
+                cudaGetLastError();
+                b->adj_refused = need;
+            }
+        }
+        if (b->adj_bytes >= need) C = T;
+    }
+    const size_t need = bytes_for(C);
+    if (b->adj_bytes < need) {
         if (b->adj_mem) cudaFree(b->adj_mem);
         b->adj_mem = nullptr;
         b->adj_bytes = 0;
-        if (cudaMalloc(&b->adj_mem, need) == cudaSuccess) {
-            b->adj_bytes = need;
-            break;
+        if (cudaMalloc(&b->adj_mem, need) != cudaSuccess) {
+            cudaGetLastError();
+            b->adj_mem = nullptr;
+            set_error("adjoint work memory (" + std::to_string(need >> 20) + " MiB) could not be allocated; "
+                      "use a larger checkpoint interval or fewer filters per handle");
+            return MCKL_B200_ERR_NOMEM;
         }
-        cudaGetLastError();
-        b->adj_mem = nullptr;
-        if (C > static_cast<uint64_t>(checkpoint_every)) {
-            C = static_cast<uint64_t>(checkpoint_every);
-            continue;
-        }
-        set_error("adjoint work memory (" + std::to_string(need >> 20) + " MiB) could not be allocated; "
-                  "use a larger checkpoint interval or fewer filters per handle");
-        return MCKL_B200_ERR_NOMEM;
+        b->adj_bytes = need;
     }
     const uint64_t nck = C >= T ? 1 : T / C + 1;
     char *p = static_cast<char *>(b->adj_mem);

@@ -47,3 +47,23 @@ def test_a_given_interval_bounds_the_memory():
     b.close()
     for ll, g in out[1:]:
         assert np.array_equal(ll, out[0][0]) and np.array_equal(g, out[0][1])
+
+
+def test_records_that_do_not_fit_leave_the_memory_alone():
+    require_cuda()
+    import mckl_b200 as mb
+
+    b = handle(mb)
+    want = b.adjoint(checkpoint_every=80)  # takes more than the default's checkpoints would
+    # leave less than the whole run's records and more than nothing
+    free = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free - formula(32), dtype=torch.uint8, device="cuda")
+    try:
+        for _ in range(2):
+            n, (ll, g) = used(lambda: b.adjoint())
+            assert n == 0, n
+            assert np.array_equal(ll, want[0]) and np.array_equal(g, want[1])
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+        b.close()
