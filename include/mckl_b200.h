@@ -295,15 +295,17 @@ int mckl_b200_batched_adjoint_records(mckl_b200_batched_t *b, int checkpoint_eve
 
 /* Score estimate by the Fisher identity (no counterpart in the reference):
  * grad log p(y_1:T | theta) = E[grad log p(x_0:T, y_1:T | theta) | y_1:T],
- * estimated in the same forward pass as each filter's FP64 log-likelihood by
- * PaRIS (per-particle statistics updated from two backward draws per step, an
+ * estimated in the same forward pass as each filter's FP64 log-likelihood
+ * (mckl_b200_batched_run's with the handle's block shape, bit for bit) by PaRIS (per-particle statistics updated from two backward draws per step, an
  * independent Metropolis-Hastings chain started at the particle's ancestor).
  * Unlike the adjoint, which differentiates the estimate with the ancestors
  * held fixed, this is a consistent estimate of the exact score: its error
  * against the Kalman gradient is Monte Carlo error that falls as N grows.
  * Handle created with fp64 = 1.  loglik: F doubles (may be NULL), score:
  * F x 3 doubles (d/dphi, d/dsx, d/dsy), HOST arrays; synchronizes `stream`.
- * Device memory: 80 B x the largest N per SM. */
+ * Device memory, kept by the handle, for each CTA (one per filter, at most one
+ * per SM): 72 B x the largest N, and 20 B x N more where the cloud does not fit
+ * in shared memory (N above 10616; 9682 with 1024 threads). */
 int mckl_b200_batched_score(mckl_b200_batched_t *b, double *loglik, double *score, void *stream);
 
 /* Autotuner: times the candidate block shapes (threads per CTA x resident CTAs

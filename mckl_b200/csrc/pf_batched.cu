@@ -354,7 +354,11 @@ __device__ __forceinline__ bool log_less(uint32_t w, double lr)
 // particle) and the slots' parents fit in shared memory they are read from
 // there.  The acceptance tests take a double logarithm only where a
 // single-precision one cannot decide.
-template <int THREADS, bool SMEM>
+//
+// SUMS: the threads of the handle's block shape, whose order the step's sums keep,
+// so that the log-likelihood and the resampling decisions are those of the handle's
+// run() bit for bit.
+template <int SUMS, int THREADS, bool SMEM>
 __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *filt, const int *order, int nf,
     const double *y, int T, double threshold, double *xa, double *xb, double *lw, uint32_t *scanS, uint32_t *epos,
     double *loglik, uint32_t *nresampled, int *queue, ScoreArgs A)
@@ -388,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_pf_score(const BatchedFilter *fi
         const double isx2 = 1.0 / (sx * sx), hsx2 = 0.5 * isx2;
         const double q0 = 1.0 - phi * phi, isd02 = q0 * isx2;
         const PhiloxGen gb{F.rkey[0], F.rkey[1] ^ 0x9E3779B9u};
-        FilterRun<double, THREADS, false> run;
+        FilterRun<double, THREADS, false, Ar1Model, SUMS> run;
         run.setup(F, xa, xb, lw, scanS, epos, nullptr, nullptr, nullptr, threshold);
         // t = 0: the initial cloud, equal weights, no resampling
         run.step(0, yf[0], shd, shd, shu, shj);
@@ -614,44 +618,64 @@ int pf_adjoint_launch(const BatchedArgs &a, const int *order, int nf, int thread
     }
 }
 
-// The score's block shape is its own: 512 threads (128 registers: the eight
-// proposals of a particle are in flight at once), one CTA per SM.  256 filters
-// x 8192 particles x 100 steps (one B200): 57.7 ms with the dependent reads and
-// 256-thread CTAs; with the independent reads 36.7 / 28.1 / 37.0 ms at 256
+// The score kernel's CTAs: 512 threads (128 registers: the eight proposals of a
+// particle are in flight at once), 1024 for handles of 1024, one CTA per SM.  256
+// filters x 8192 particles x 100 steps (one B200): 57.7 ms with the dependent reads
+// and 256-thread CTAs; with the independent reads 36.7 / 28.1 / 37.0 ms at 256
 // threads x 1 / 2 / 4 CTAs per SM, 25.2 / 26.8 at 512 x 1 / 2, 26.5 at 1024 x 1;
-// 21.9 ms at 512 x 1 with the cloud in shared memory.
-constexpr int kScoreThreads = 512;
-// shared memory left for the cloud beside the step's own
-constexpr size_t kScoreDyn = 227 * 1024 - 4 * shj_words<kScoreThreads>() - 1024;
-constexpr size_t kScoreCloudBytes = sizeof(double2) + sizeof(uint32_t);
-
-// Whether a cloud of n particles is kept in shared memory (up to about 10 400).
-bool score_in_smem(uint64_t n)
+// 21.9 ms at 512 x 1 with the cloud in shared memory; 22.9 with the sums of a
+// 256-thread handle (25.2 with its whole step on 256 of the threads).
+constexpr int score_block(int threads)
 {
-    return n * kScoreCloudBytes <= kScoreDyn;
+    return std::max(threads, 512);
 }
 
-template <bool SMEM>
+// shared memory left for the cloud beside the step's own
+constexpr size_t score_dyn(int threads)
+{
+    return 227 * 1024 - 4 * (threads > 512 ? shj_words<1024>() : shj_words<512>()) - 1024;
+}
+
+constexpr size_t kScoreCloudBytes = sizeof(double2) + sizeof(uint32_t);
+
+// Whether a cloud of n particles is kept in shared memory (up to 10,616; 9,682 in
+// handles of 1024 threads).
+bool score_in_smem(uint64_t n, int threads)
+{
+    return n * kScoreCloudBytes <= score_dyn(threads);
+}
+
+template <int SUMS, bool SMEM>
 int score_one(const BatchedArgs &a, const int *order, int nf, int *queue, const ScoreArgs &A, int ctas,
     cudaStream_t s)
 {
+    constexpr int THREADS = score_block(SUMS);
     const int dyn = SMEM ? static_cast<int>(A.nmax * kScoreCloudBytes) : 0;
     if (dyn)
-        MB_CUDA(cudaFuncSetAttribute(k_pf_score<kScoreThreads, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(kScoreDyn)));
-    k_pf_score<kScoreThreads, SMEM><<<ctas, kScoreThreads, dyn, s>>>(a.filt, order, nf, a.y, a.T, a.threshold,
+        MB_CUDA(cudaFuncSetAttribute(k_pf_score<SUMS, THREADS, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            static_cast<int>(score_dyn(THREADS))));
+    k_pf_score<SUMS, THREADS, SMEM><<<ctas, THREADS, dyn, s>>>(a.filt, order, nf, a.y, a.T, a.threshold,
         static_cast<double *>(a.xa), static_cast<double *>(a.xb), static_cast<double *>(a.lw), a.scanS, a.epos,
         a.loglik, a.nresampled, queue, A);
     MB_LAUNCH_CHECK();
     return MCKL_B200_OK;
 }
 
-int pf_score_launch(const BatchedArgs &a, const int *order, int nf, int *queue, const ScoreArgs &A, int ctas,
-    cudaStream_t s)
+int pf_score_launch(const BatchedArgs &a, const int *order, int nf, int threads, int *queue, const ScoreArgs &A,
+    int ctas, cudaStream_t s)
 {
     MB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), s));
-    return score_in_smem(A.nmax) ? score_one<true>(a, order, nf, queue, A, ctas, s)
-                                 : score_one<false>(a, order, nf, queue, A, ctas, s);
+    const auto launch = [&](auto t) {
+        constexpr int SUMS = decltype(t)::value;
+        return score_in_smem(A.nmax, SUMS) ? score_one<SUMS, true>(a, order, nf, queue, A, ctas, s)
+                                           : score_one<SUMS, false>(a, order, nf, queue, A, ctas, s);
+    };
+    switch (threads) {
+        case 128: return launch(std::integral_constant<int, 128>{});
+        case 256: return launch(std::integral_constant<int, 256>{});
+        case 512: return launch(std::integral_constant<int, 512>{});
+        default: return launch(std::integral_constant<int, 1024>{});
+    }
 }
 
 // The filters that a cluster runs (the first of the sorted ones) and their share
@@ -1170,7 +1194,7 @@ int mckl_b200_batched_score(mckl_b200_batched_t *b, double *loglik, double *scor
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int ctas = std::max(1, std::min(b->F, sms));
-    const uint64_t nm = b->nmax, ng = score_in_smem(nm) ? 0 : nm;  // ng: particles of the cloud in global memory
+    const uint64_t nm = b->nmax, ng = score_in_smem(nm, b->threads) ? 0 : nm;  // ng: particles of the cloud in global memory
     const size_t need = align256(ctas * nm * 8) + align256(ctas * ng * sizeof(double2)) +
                         align256(ctas * ng * 4) + align256(ctas * 2 * nm * sizeof(ScoreTau)) +
                         align256(static_cast<size_t>(b->F) * 24);
@@ -1197,7 +1221,7 @@ int mckl_b200_batched_score(mckl_b200_batched_t *b, double *loglik, double *scor
     A.anc = reinterpret_cast<uint32_t *>(take(ctas * ng * 4));
     A.tau = reinterpret_cast<ScoreTau *>(take(ctas * 2 * nm * sizeof(ScoreTau)));
     A.score = reinterpret_cast<double *>(take(static_cast<size_t>(b->F) * 24));
-    int rc = pf_score_launch(b->a, b->order, b->F, b->queue, A, ctas, s);
+    int rc = pf_score_launch(b->a, b->order, b->F, b->threads, b->queue, A, ctas, s);
     if (rc != MCKL_B200_OK) return rc;
     if (loglik) MB_CUDA(cudaMemcpyAsync(loglik, b->a.loglik, b->F * 8, cudaMemcpyDeviceToHost, s));
     MB_CUDA(cudaMemcpyAsync(score, A.score, static_cast<size_t>(b->F) * 24, cudaMemcpyDeviceToHost, s));

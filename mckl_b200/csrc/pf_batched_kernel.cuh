@@ -602,7 +602,12 @@ __device__ __forceinline__ void cluster_store(T *p, uint32_t rank, T v)
 // Monte Carlo divergence a flipped ancestor would otherwise start; with
 // R = double and perturbed parameters it is the common-random-numbers,
 // fixed-ancestor evaluation that finite differences of the estimate need.
-template <typename R, int THREADS, bool SHADOW, class Model = Ar1Model>
+//
+// SUMS < THREADS: the normaliser's sums, whose bits depend on which thread meets
+// which unit, are formed by the first SUMS threads as a CTA of SUMS threads forms
+// them, from the log-weights that all THREADS have written.  (The rest of the step
+// does not depend on the number of threads.)
+template <typename R, int THREADS, bool SHADOW, class Model = Ar1Model, int SUMS = THREADS>
 struct FilterRun {
     NoiseLayout lay;
     PhiloxGen gm, gr;
@@ -714,7 +719,7 @@ struct FilterRun {
             lay.words(gm, u, src, wr, wa);
             st.load4(pa, pb, lo, hi, old);
             st.move4(wr, wa, pa, pb, lo, hi, old, v, vs);
-            if (t > 0) {
+            if (SUMS == THREADS && t > 0) {
                 acc.add(v, 2 * lo, 2 * hi);
                 if constexpr (SHADOW) accs.add(vs, 2 * lo, 2 * hi);
             }
@@ -728,7 +733,7 @@ struct FilterRun {
             if constexpr (SHADOW)
                 st.one_shadow(__dmul_rn(Math<double>::radius(u01oc<double>(w0)), Math<double>::cos2pi(u01oc<double>(w1))),
                     N - 1, vs[0]);
-            if (t > 0) {
+            if (SUMS == THREADS && t > 0) {
                 acc.add(v, 0, 1);
                 if constexpr (SHADOW) accs.add(vs, 0, 1);
             }
@@ -736,6 +741,31 @@ struct FilterRun {
         if (t == 0) {
             __syncthreads();
             return false;
+        }
+        if constexpr (SUMS < THREADS) {
+            static_assert(!SHADOW, "the shadow's sums are not formed here");
+            __syncthreads();
+            if (threadIdx.x < SUMS) {
+                for (uint32_t u = threadIdx.x; u < static_cast<uint32_t>(lay.units); u += SUMS) {
+                    R v[8];
+                    int lo, hi;
+                    uint32_t pa[4], pb[4];
+                    uint64_t src;
+                    lay.slots(t, u, pa, pb, &lo, &hi, &src);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (j >= lo && j < hi) {
+                            v[2 * j] = st.l[pa[j]];
+                            v[2 * j + 1] = st.l[pb[j]];
+                        }
+                    }
+                    acc.add(v, 2 * lo, 2 * hi);
+                }
+                if ((N & 1) && threadIdx.x == SUMS - 1) {
+                    const R v[1] = {st.l[N - 1]};
+                    acc.add(v, 0, 1);
+                }
+            }
         }
         // ---- FP64 normaliser: S = sum exp(l - M), Q = sum exp^2; the log
         // normaliser of the weights relative to M is carried to the next step,
