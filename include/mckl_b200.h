@@ -321,6 +321,10 @@ int mckl_b200_batched_autotune(mckl_b200_batched_t *b, int max_trials, int *thre
 int mckl_b200_batched_set_y(mckl_b200_batched_t *b, const double *y, void *stream);
 /* The block shape the handle runs with (set by _config or the autotuner). */
 int mckl_b200_batched_get_config(const mckl_b200_batched_t *b, int *threads, int *ctas_per_sm);
+/* How many of the handle's filters, the largest first, a run gives to a cluster
+ * of four CTAs each (diagnostics; the results do not depend on it).  FP32 handles
+ * without a shadow: the filters that alone would outlast the rest of the batch. */
+int mckl_b200_batched_cluster_filters(const mckl_b200_batched_t *b, int *n);
 int mckl_b200_batched_destroy(mckl_b200_batched_t *b);
 
 /* Sequential left fold s_i = s_{i-1} + x_i (s_{-1} = s0) of n nonnegative

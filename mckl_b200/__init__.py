@@ -197,6 +197,7 @@ _bt_shadow = _bind("mckl_b200_batched_shadow", [_vp, _vp, _vp])
 _bt_set_y = _bind("mckl_b200_batched_set_y", [_vp, _vp, _vp])
 _bt_autotune = _bind("mckl_b200_batched_autotune", [_vp, _i, _vp, _vp, _vp, _vp, _vp])
 _bt_get_config = _bind("mckl_b200_batched_get_config", [_vp, _vp, _vp])
+_bt_cluster_filters = _bind("mckl_b200_batched_cluster_filters", [_vp, _vp])
 _bt_shadow_params = _bind("mckl_b200_batched_shadow_params", [_vp, _vp, _vp, _vp])
 _bt_adjoint = _bind("mckl_b200_batched_adjoint_records", [_vp, _i, _sz, _vp, _vp, _vp])
 _bt_score = _bind("mckl_b200_batched_score", [_vp, _vp, _vp, _vp])
@@ -273,6 +274,12 @@ class BatchedFilters:
         t, c = ctypes.c_int(), ctypes.c_int()
         _check(_bt_get_config(self.h, ctypes.byref(t), ctypes.byref(c)))
         return (t.value, c.value)
+
+    def cluster_filters(self):
+        """How many of the filters a run gives to a cluster of CTAs each."""
+        n = ctypes.c_int()
+        _check(_bt_cluster_filters(self.h, ctypes.byref(n)))
+        return n.value
 
     def set_shadow_params(self, phi, sx, sy):
         """Parameters of the FP64 shadow (handles made with shadow=True)."""

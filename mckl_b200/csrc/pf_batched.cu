@@ -926,6 +926,17 @@ int mckl_b200_batched_get_config(const mckl_b200_batched_t *b, int *threads, int
     return MCKL_B200_OK;
 }
 
+int mckl_b200_batched_cluster_filters(const mckl_b200_batched_t *b, int *n)
+{
+    MB_CHECK_ARG(b != nullptr && n != nullptr, "null argument");
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    double share = 0.0;
+    *n = b->a.terms ? joint_filters(b->sorted.data(), b->F, sms * b->ctas_per_sm, &share) : 0;
+    return MCKL_B200_OK;
+}
+
 int mckl_b200_batched_run(mckl_b200_batched_t *b, void *stream)
 {
     MB_CHECK_ARG(b != nullptr, "null handle");
