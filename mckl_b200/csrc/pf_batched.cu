@@ -31,6 +31,7 @@
 #include "block_scan.cuh"
 #include "common.cuh"
 #include "pf_batched.cuh"
+#include "crmathf.cuh"
 #include "pf_batched_kernel.cuh"
 
 namespace mckl_b200 {
@@ -334,19 +335,6 @@ struct ScoreArgs {
     ScoreTau *tau;         // 2 x nmax per CTA
     double *score;         // 3 per filter
 };
-
-// log(u) < lr for u = (w + 1/2) 2^-32, as the double logarithm decides it.
-// The single-precision logarithm of u is within 1e-5 of log u (rounding u:
-// 2^-23 relative; __logf: 2^-21.4 absolute for u in [0.5, 1], 3 ulps of at most
-// 23 below), so it decides whenever lr is further away than that (rounding lr
-// to float is below 2e-6 for |lr| <= 32); a NaN goes to the double comparison.
-__device__ __forceinline__ bool log_less(uint32_t w, double lr)
-{
-    const float u = __fmul_rn(__fadd_rn(__uint2float_rn(w), 0.5f), 0x1p-32f);
-    const float d = __fsub_rn(__double2float_rn(lr), __logf(u));
-    if (fabsf(d) > 1e-4f) return d > 0.0f;
-    return log((static_cast<double>(w) + 0.5) * 0x1p-32) < lr;
-}
 
 // What bounds it: the latency of the backward draws' random reads.  The
 // proposals of a particle's eight moves do not depend on the chain's state, so
