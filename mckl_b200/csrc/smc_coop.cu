@@ -342,7 +342,8 @@ struct Tiling {
 
 Tiling tiling(uint64_t n)
 {
-    static constexpr int kShapes[][2] = {{512, 2}, {1024, 4}, {1024, 7}, {1024, 8}};
+    static constexpr int kShapes[][2] = {{512, 2}, {512, 4}, {1024, 3}, {1024, 4}, {1024, 5}, {1024, 6}, {1024, 7},
+        {1024, 8}};
     for (const auto &k : kShapes) {
         const uint64_t tile = static_cast<uint64_t>(k[0]) * k[1], T = (n + tile - 1) / tile;
         if (T <= kMaxTiles) return {k[0], k[1], static_cast<unsigned>(T)};
@@ -414,11 +415,15 @@ int launch(K kernel, int threads, size_t dyn, std::atomic<int> *cache, unsigned 
         return launch(KERNEL<THR, PER>, THR, sizeof(TileMem<THR * PER>), cache_[SLOT], (TILING).T, STREAM, __VA_ARGS__);
 #define COOP_LAUNCH(KERNEL, TILING, STREAM, ...)                          \
     [&]() -> int {                                                        \
-        static std::atomic<int> cache_[4][16];                            \
+        static std::atomic<int> cache_[8][16];                            \
         COOP_SHAPE(KERNEL, 512, 2, 0, TILING, STREAM, __VA_ARGS__)        \
-        COOP_SHAPE(KERNEL, 1024, 4, 1, TILING, STREAM, __VA_ARGS__)       \
-        COOP_SHAPE(KERNEL, 1024, 7, 2, TILING, STREAM, __VA_ARGS__)       \
-        COOP_SHAPE(KERNEL, 1024, 8, 3, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 512, 4, 1, TILING, STREAM, __VA_ARGS__)        \
+        COOP_SHAPE(KERNEL, 1024, 3, 2, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 4, 3, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 5, 4, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 6, 5, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 7, 6, TILING, STREAM, __VA_ARGS__)       \
+        COOP_SHAPE(KERNEL, 1024, 8, 7, TILING, STREAM, __VA_ARGS__)       \
         return kCoopNo;                                                   \
     }()
 

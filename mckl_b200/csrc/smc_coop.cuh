@@ -18,12 +18,22 @@
 // loop over a thread's elements is rolled (with the loops unrolled and the
 // values in registers the weight call of 1001 particles took 56 us).
 //
-// Tiles: THR threads of PER consecutive elements each, at most one tile per SM.
-// 512 x 2 while that many tiles of 1024 do (one CTA alone up to 1024 elements, a
-// cluster up to 8192), since more CTAs shorten every phase; then 1024 x 4, 7 or 8,
-// so that every SM has the same work (2^20 particles on 256 tiles of 4096, two
-// on most SMs: 97 us a filter step; on 147 tiles of 7168: 91 us).  Clouds of
-// more tiles than that take the multi-kernel step.
+// Tiles: THR threads of PER consecutive elements each, at most one tile per SM:
+// the smallest tile that fits the cloud on 148 SMs, in steps of 1024 elements up to
+// 8192 (one CTA alone up to 1024 elements, a cluster up to 8192), since more CTAs
+// shorten every phase and equal ones wait least for each other.  On a B200, a step
+// of the plain systematic and multinomial filters (T = 20):
+//   particles   multi-kernel     512 x 2, 1024 x 4, 7, 8   every 1024 elements
+//   151,553     157 / 167 us     67 / 110 us (38 tiles)    54 /  92 us (74 tiles)
+//   300,000     162 / 174        70 / 117                  58 /  99
+//   380,000     165 / 179        71 / 119                  67 / 105
+//   500,000     174 / 185        73 / 119                  73 / 120 (the same)
+//   606,209     183 / 199        91 / 173 (85 tiles)       81 / 142 (119 tiles)
+//   800,000     194 / 214        90 / 175                  84 / 156
+//   1,048,576   214 / 232        93 / 177                  92 / 178 (the same)
+// (2^20 particles on 256 tiles of 4096, two on most SMs: 97 us a systematic step.)
+// Multinomial counts of 606,209 particles alone: 147 us multi-kernel, 144 to 152 on
+// 85 tiles, 118 on 119.  Clouds of more tiles than SMs take the multi-kernel step.
 #pragma once
 
 #include <cstdint>
