@@ -738,11 +738,20 @@ __device__ __forceinline__ void gamma_stream(const G &g, const GammaParam<R> &k,
 //
 // A call of one stream runs on one SM, chunk after chunk, and takes 1024 threads
 // there (100,000 values, Threefry, single precision, shapes 0.3 / 2.5: 445 / 432 us
-// with 256 threads and unrolled loops, 317 / 315 now).
+// with 256 threads and unrolled loops, 317 / 315 now).  A short one takes 256
+// threads with registers for no more than one CTA: 1024 threads have 64 each, their
+// barriers and, with Threefry's 64-bit rounds, spilled registers cost more than the
+// warps bring.  Whole calls, Threefry / ARS, alpha = 1, single precision: 10
+// values 44 / 45 us with 1024 threads, 34 / 37 with 256; 1000 values 44 / 45, 36 /
+// 43; 2048 values 44 / 45, 36 / 45; alpha = 0.3, 2048 values of Threefry 69, 61, of
+// Philox 57 and 58, 8000 values 69 and 72.
 constexpr int kGammaThreads = 256, kGammaOneThreads = 1024;
 
-template <class G, typename W, typename R, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_gamma(G g, Ctr ctr0, uint32_t idx0, int blocks, uint64_t nstreams,
+template <class G>
+constexpr uint64_t kGammaShort = G::kWords == 8 ? 2048 : 1024;  // longest call on 256 threads (Threefry: 8 words)
+
+template <class G, typename W, typename R, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) k_gamma(G g, Ctr ctr0, uint32_t idx0, int blocks, uint64_t nstreams,
     const uint32_t *list, uint64_t n, const GammaParam<R> *params, R *r, Ctr *ctr_out, uint32_t *idx_out)
 {
     constexpr uint32_t M = static_cast<uint32_t>(GammaSmem<G, W, R>::WPB);
@@ -807,9 +816,9 @@ int gamma_impl(mckl_b200_engine_t *e, bool blocks, size_t nstreams, size_t n, co
         using G = decltype(g);
         auto run = [&](auto wtag) {
             using W = decltype(wtag);
-            auto launch = [&](auto threads) {
+            auto launch = [&](auto threads, auto ctas) {
                 constexpr int T = decltype(threads)::value;
-                auto kern = k_gamma<G, W, R, T>;
+                auto kern = k_gamma<G, W, R, T, decltype(ctas)::value>;
                 const int dyn = G::kDynSmem + GammaSmem<G, W, R>::kBytes;
                 MB_CUDA(allow_dyn_smem(kern, dyn));
                 kern<<<static_cast<unsigned>(std::min<uint64_t>(nstreams, 0x7fffffffu)), T, dyn, s>>>(g, c0, idx0,
@@ -817,8 +826,11 @@ int gamma_impl(mckl_b200_engine_t *e, bool blocks, size_t nstreams, size_t n, co
                 MB_LAUNCH_CHECK();
                 return static_cast<int>(MCKL_B200_OK);
             };
-            if (blocks) return launch(std::integral_constant<int, kGammaThreads>{});
-            return launch(std::integral_constant<int, kGammaOneThreads>{});
+            constexpr std::integral_constant<int, kGammaThreads> t;
+            constexpr std::integral_constant<int, 1> one;
+            if (blocks) return launch(t, std::integral_constant<int, 1024 / kGammaThreads>{});
+            if (n <= kGammaShort<G>) return launch(t, one);
+            return launch(std::integral_constant<int, kGammaOneThreads>{}, one);
         };
         if (w64) return run(uint64_t{});
         return run(uint32_t{});
