@@ -7,7 +7,7 @@
 //   * aligned: the stream starts on a block boundary and the output is
 //     16-byte aligned -> each thread turns whole blocks into 128-bit stores,
 //     the values of a last partial block in the same launch;
-//   * shifted: 4096 values or more from the middle of a block into a 16-byte
+//   * shifted: many values (launch_words) from the middle of a block into a 16-byte
 //     aligned output -> the same stores, the values shifted between lanes;
 //   * staged: short calls and other alignments -> a CTA generates a tile of
 //     blocks into shared memory and writes its outputs from there, coalesced.
@@ -601,9 +601,18 @@ static int launch_words(const G &g, const Ctr &B, uint32_t off, uint64_t n, type
         return MCKL_B200_OK;
     }
     if constexpr (F::kIn == 1) {
-        // enough groups for the shifted shape to pay for its last partial warp
-        if (reinterpret_cast<uintptr_t>(out) % 16 == 0 && n >= 4096) {
-            const uint64_t ng = n / WPB, warps = (ng + 1 + 30) / 31;
+        // Where the shifted shape is the faster one.  ARS sets up four tables per SM
+        // for it, which pays once the staged shape has a third tile for an SM:
+        // words, staged / shifted, 30,000 blocks 3.8 / 4.7 us, 70,000 5.2 / 4.9,
+        // 75,776 6.2 / 4.9, 200,000 9.9 / 6.5; double Exponentials 5.8 / 7.5, 6.8 /
+        // 7.6, 8.5 / 7.6, 12.6 / 11.3.  The others from 4096 values: Philox words
+        // 1.8 / 1.5 us, 10^6 3.9 / 2.9; double Exponentials 3.2 / 3.1, 7.6 / 7.3;
+        // Threefry's 4.8 / 4.6, 9.4 / 9.3 (below 2000 values 4.4 against 3.1).
+        const uint64_t ng = n / WPB;
+        const bool enough =
+            std::is_same<G, ArsGen>::value ? ng >= 2 * 256 * static_cast<uint64_t>(sm_count()) : n >= 4096;
+        if (reinterpret_cast<uintptr_t>(out) % 16 == 0 && enough) {
+            const uint64_t warps = (ng + 1 + 30) / 31;
             const uint32_t rem = static_cast<uint32_t>(n % WPB);
             if constexpr (std::is_same<G, ArsGen>::value) {
                 MB_CUDA(allow_dyn_smem(k_shifted<ArsGen4, W, F, 1024>, ArsGen4::kDynSmem));
@@ -712,7 +721,11 @@ static int normal_impl(mckl_b200_engine_t *e, size_t n, R *r, R mean, R sd, void
                 MB_LAUNCH_CHECK();
                 return static_cast<int>(MCKL_B200_OK);
             };
-            // a chunk or two per SM: its latency counts, one pair per thread
+            // A chunk or two per SM: its latency counts, one pair per thread.  Device
+            // time with 512 / 128 threads (ARS: 256), 148, 296 and 444 chunks, double:
+            // Philox 5.5 / 6.5, 6.9 / 6.8, 9.0 / 7.8 us, Threefry 5.7 / 7.1, 7.3 / 7.3,
+            // 11.1 / 7.9, ARS 7.4 / 7.7, 9.6 / 9.5, 12.2 / 11.7; single: Philox 2.6 /
+            // 3.9, 3.4 / 4.2, 4.2 / 4.6.
             if (chunks <= 2 * static_cast<uint64_t>(sm_count())) return launch(std::integral_constant<int, 512>{});
             return launch(std::integral_constant<int, G::kDynSmem ? 256 : 128>{});
         };
