@@ -465,7 +465,9 @@ __global__ void __launch_bounds__(256) k_staged(G g, Ctr base, uint32_t off, uin
 // the generator keeps a table per CTA) wait less at the two barriers of a chunk;
 // calls of few chunks run 512 threads on each.
 // 2^24 + 1 values (Threefry): 176.0 us before, 133.3 now (one CTA size
-// of 256 threads and no list: 173.2).
+// of 256 threads and no list: 173.2).  Single precision has no list and a loop of its
+// own: through the list's loop, with whole indices for every store, 2^24 values
+// took 46.3 / 62.3 us (Philox / Threefry) against 44.2 / 60.0.
 // ---------------------------------------------------------------------------
 template <class G, typename W, typename R, int K, int THREADS>
 __global__ void __launch_bounds__(THREADS) k_normal(G g, Ctr base, uint32_t off, uint64_t nchunks, uint32_t last_len,
@@ -523,7 +525,23 @@ __global__ void __launch_bounds__(THREADS) k_normal(G g, Ctr base, uint32_t off,
         }
         __syncthreads();
         const uint64_t o = c * K;
-        for (uint32_t p0 = warp * 32; p0 < nu; p0 += THREADS) {
+        if constexpr (!kDefer) {
+            R *oc = out + o;
+            for (uint32_t p = threadIdx.x; p < nu; p += THREADS) {
+                R s, sn, cs;
+                pair_quick(O::u01(kOC, st[s0 + p]), O::mul(O::kTwoPi, O::u01(kOC, st[s0 + nu + p])), &s, &sn, &cs);
+                s = O::sqrt(O::mul(static_cast<R>(-2), s));
+                if (sd != static_cast<R>(1)) s = O::mul(sd, s);
+                if (mean != static_cast<R>(0)) {
+                    oc[p] = O::fma(s, sn, mean);
+                    oc[nu + p] = O::fma(s, cs, mean);
+                } else {
+                    oc[p] = O::mul(s, sn);
+                    oc[nu + p] = O::mul(s, cs);
+                }
+            }
+        }
+        for (uint32_t p0 = kDefer ? warp * 32 : nu; p0 < nu; p0 += THREADS) {
             const uint32_t p = p0 + lane;
             bool ok = true;
             if (p < nu) {
