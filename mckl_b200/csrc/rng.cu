@@ -353,8 +353,7 @@ __global__ void __launch_bounds__(256) k_blocks_plo(PhiloxLo p, uint32_t nblk, u
 // of two with shuffles and store whole vectors.  A warp's last lane only serves
 // the one before it (31 groups for 32 blocks).  Against the staged shape: no
 // shared memory, no barriers, vector stores (5e6 single-precision Exponentials
-// from ARS at an offset of one word: 31.0 -> 24.6 us, with the wider table
-// set-up).
+// from ARS at an offset of one word: 31.0 -> 23.2 us).
 template <class G, typename W, class F, int THREADS = 256>
 __global__ void __launch_bounds__(THREADS) k_shifted(G g, Ctr base, uint32_t off, uint64_t ngroups,
     uint32_t rem, typename F::out_t *out, F f)
@@ -620,8 +619,8 @@ static int launch_words(const G &g, const Ctr &B, uint32_t off, uint64_t n, type
     }
     if constexpr (F::kIn == 1) {
         // Where the shifted shape is the faster one.  ARS sets up four tables per SM
-        // for it, which pays once the staged shape has a third tile for an SM:
-        // words, staged / shifted, 30,000 blocks 3.8 / 4.7 us, 70,000 5.2 / 4.9,
+        // for it, which pays once the staged shape has a third tile for an SM: words
+        // (measured with a table set-up 0.5 us longer), staged / shifted, 30,000 blocks 3.8 / 4.7 us, 70,000 5.2 / 4.9,
         // 75,776 6.2 / 4.9, 200,000 9.9 / 6.5; double Exponentials 5.8 / 7.5, 6.8 /
         // 7.6, 8.5 / 7.6, 12.6 / 11.3.  The others from 4096 values: Philox words
         // 1.8 / 1.5 us, 10^6 3.9 / 2.9; double Exponentials 3.2 / 3.1, 7.6 / 7.3;
