@@ -584,7 +584,9 @@ static int launch_words(const G &g, const Ctr &B, uint32_t off, uint64_t n, type
     if (n == 0) return MCKL_B200_OK;
     constexpr int WPB = G::kWords / WordView<W>::kPer32;
     constexpr int OPB = WPB / F::kIn;
-    const bool aligned = (off == 0) && (reinterpret_cast<uintptr_t>(out) % 16 == 0);
+    // (a call of less than one block is staged: one to three double Exponentials of
+    // Threefry 2.6 us on the device, 3.9 by a thread that transforms a whole block)
+    const bool aligned = (off == 0) && n >= OPB && (reinterpret_cast<uintptr_t>(out) % 16 == 0);
     // ARS: 32 KiB of table per CTA bounds residency at 6 CTAs per SM
     const int ctas = std::is_same<G, ArsGen>::value ? 6 : 8;
     if (aligned) {
@@ -620,11 +622,12 @@ static int launch_words(const G &g, const Ctr &B, uint32_t off, uint64_t n, type
     if constexpr (F::kIn == 1) {
         // Where the shifted shape is the faster one.  ARS sets up four tables per SM
         // for it, which pays once the staged shape has a third tile for an SM: words
-        // (measured with a table set-up 0.5 us longer), staged / shifted, 30,000 blocks 3.8 / 4.7 us, 70,000 5.2 / 4.9,
-        // 75,776 6.2 / 4.9, 200,000 9.9 / 6.5; double Exponentials 5.8 / 7.5, 6.8 /
-        // 7.6, 8.5 / 7.6, 12.6 / 11.3.  The others from 4096 values: Philox words
-        // 1.8 / 1.5 us, 10^6 3.9 / 2.9; double Exponentials 3.2 / 3.1, 7.6 / 7.3;
-        // Threefry's 4.8 / 4.6, 9.4 / 9.3 (below 2000 values 4.4 against 3.1).
+        // (measured with a table set-up 0.5 us longer), staged / shifted, 30,000
+        // blocks 3.8 / 4.7 us, 70,000 5.2 / 4.9, 75,776 6.2 / 4.9, 200,000 9.9 / 6.5;
+        // double Exponentials 5.8 / 7.5, 6.8 / 7.6, 8.5 / 7.6, 12.6 / 11.3.  The
+        // others from 4096 values: Philox words 1.8 / 1.5 us, 10^6 3.9 / 2.9; double
+        // Exponentials 3.2 / 3.1, 7.6 / 7.3; Threefry's 4.8 / 4.6, 9.4 / 9.3 (500
+        // values 3.1 / 4.4).
         const uint64_t ng = n / WPB;
         const bool enough =
             std::is_same<G, ArsGen>::value ? ng >= 2 * 256 * static_cast<uint64_t>(sm_count()) : n >= 4096;
