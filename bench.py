@@ -435,7 +435,7 @@ def bench_plain_c3(N=1 << 20, T=1000):
             "scan_ties_note": "uniforms within one representable step of a cumulative weight, over all resampling "
                               "steps; the cumulative weights are the reference's sequential fold bit for bit, so "
                               "a tie flips no ancestor",
-            "bound": "latency: per step the exchanges between 148 tiles of the exact sequential folds, in cooperative "
+            "bound": "latency: per step the exchanges between 147 tiles of the exact sequential folds, in cooperative "
                      "kernels that take the resampling decisions on the device",
             "y": y}
 

@@ -200,7 +200,9 @@ int mckl_b200_select_f32(size_t N, size_t dim, const uint64_t *idx_dev, float *s
  * t of log sum_i W_{t-1,i} p(y_t | x_{t,i}).  ess_hist / resampled (host,
  * T + 1 entries) and anc_dev ((T + 1) x N parent indices, rows written at
  * resampling steps) are optional.  x_dev, W_dev (device, N) receive the final
- * particles and weights.  Synchronizes once per step. */
+ * particles and weights.  Synchronizes: once at its end for clouds of up to
+ * 148 x 8192 particles (on 148 SMs), whose steps run in one kernel, and once per
+ * step for larger ones; x_dev and W_dev are complete on return. */
 int mckl_b200_pf_ar1_plain_f64(size_t N, size_t T, const double *y, double phi, double sx, double sy, double sd0,
     const uint32_t mkey[2], const uint32_t rkey[2], int scheme, double threshold, double *loglik,
     double *ess_hist, uint8_t *resampled, uint64_t *anc_dev, double *x_dev, double *W_dev, void *stream);

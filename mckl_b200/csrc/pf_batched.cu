@@ -674,8 +674,8 @@ int pf_score_launch(const BatchedArgs &a, const int *order, int nf, int threads,
 // totals of the resampling are formed twice, and five cluster barriers wait.
 // One B200, 256 threads x 4 CTAs per SM: 1024 filters, log-uniform in
 // [256, 65536], T = 100: 42.6 ms without, 21.9 / 21.3 / 20.9 / 21.3 / 22.9 with
-// those above 0.5 / 0.75 / 1 / 1.25 / 1.5 shares (clusters of 2 and of 8: 25.4 and
-// 24.8 at one share); 300 filters up to 20000, T = 60: 5.5 -> 3.7; 24 filters up to
+// those above 0.5 / 0.75 / 1 / 1.25 / 1.5 shares (an earlier form of the step, at one
+// share, in clusters of 2 / 4 / 8: 25.4 / 22.4 / 24.8); 300 filters up to 20000, T = 60: 5.5 -> 3.7; 24 filters up to
 // 8375, T = 58: 1.85 -> 1.26.  4096 filters fill the chip by themselves: 32.6 ms
 // (T = 60) either way, 46 with those above half a share by clusters.
 int joint_filters(const uint64_t *sorted, int nf, int slots, double *share)
